@@ -251,6 +251,11 @@ int32_t mf_lunnon_collect(const mf_lunnon_plan *plan, int32_t depth, uint8_t *st
     return MF_OK;
 }
 
+// Leaves of the last row of a 2-D map with at least two rows (0: no such row).
+static int32_t last_row(const LunnonTables &t) {
+    return t.dim == 2 && t.p[0] >= 2 && t.p[1] >= 2 ? t.p[0] : 0;
+}
+
 static int upload_table(mf_lunnon_plan *plan) {
     if (plan->d_table) return MF_OK;
     int rc = ensure_device();
@@ -403,6 +408,7 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
         inst[k].n = p->t.n;
         inst[k].dim = p->t.dim;
         inst[k].start_leaf = d + 1;
+        inst[k].row = last_row(p->t);
         tables.insert(tables.end(), p->t.next.begin(), p->t.next.end());
         tables.resize((tables.size() + 15) / 16 * 16, 0);
         const uint64_t all = collect_lunnon_states(p->t, d, nullptr, 0, stride);
@@ -592,7 +598,7 @@ int32_t mf_sym_graph_create(int32_t n, int32_t start_i, int32_t stop_i, const ui
                 cudaError_t e = cudaMemsetAsync(d_nodes, 0, sizeof(uint64_t), s);
                 if (e != cudaSuccess) return e;
             }
-            return launch_sym_batched(edges, start_i, stop_i, d_cycles, num_cases, d_counts,
+            return launch_sym_batched(edges, n, start_i, stop_i, d_cycles, num_cases, d_counts,
                                       d_nodes, d_workspace, knobs, s);
         },
         out);
@@ -653,7 +659,7 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
         int d = depths ? depths[k] : -1;
         if (d < 0) d = default_lunnon_depth(p->t);
         if (d > p->t.n) d = p->t.n;
-        inst[k] = LunnonInstanceDev{uint32_t(meta.size()), p->t.n, p->t.dim, d + 1};
+        inst[k] = LunnonInstanceDev{uint32_t(meta.size()), p->t.n, p->t.dim, d + 1, last_row(p->t)};
         meta.insert(meta.end(), p->t.next.begin(), p->t.next.end());
         meta.resize((meta.size() + 15) / 16 * 16, 0);
         per_plan[k] = collect_lunnon_states(p->t, d, nullptr, 0, stride);
@@ -912,7 +918,7 @@ int32_t mf_sym_count_cases_batched(int32_t n, int32_t start_i, int32_t stop_i,
         set_error("uploading the edge pages failed");
         return MF_ERR_CUDA;
     }
-    MF_TRY_CUDA(launch_sym_batched(edges, start_i, stop_i, d_cycles, num_cases, d_counts, d_nodes,
+    MF_TRY_CUDA(launch_sym_batched(edges, n, start_i, stop_i, d_cycles, num_cases, d_counts, d_nodes,
                                    d_workspace, knobs, static_cast<cudaStream_t>(stream)));
     return MF_OK;
 }
@@ -957,7 +963,7 @@ int count_cases_host(int n, int start_i, int stop_i, const uint8_t *h_cycles, ui
                                     d_counts + num,
                                     d_work, knobs, s));
     else if (mode == 1)
-        MF_TRY_CUDA(launch_sym_batched(edges, start_i, stop_i, d_cycles, num, d_counts,
+        MF_TRY_CUDA(launch_sym_batched(edges, n, start_i, stop_i, d_cycles, num, d_counts,
                                        d_counts + num, d_work, knobs, s));
     else
         MF_TRY_CUDA(launch_sym_plain(edges, start_i, stop_i, d_cycles, num, d_counts, d_counts + num, s));

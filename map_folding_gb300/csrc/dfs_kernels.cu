@@ -33,6 +33,7 @@
 
 #include "dfs_core.cuh"
 #include "engine.hpp"
+#include "tail.cuh"
 
 namespace mf {
 namespace {
@@ -114,10 +115,76 @@ __global__ void ring_init_kernel(unsigned long long *seq, unsigned long long cap
         seq[k] = k;
 }
 
+// Row counting (tail.cuh) of the persistent kernels.
+constexpr int kTailFill = 16;    // frames that make a level full
+constexpr int kTailRoots = 28;   // lanes at the row that start a count
+constexpr uint32_t kTailRounds = 8;  // bookkeeping rounds that a count stands for
+constexpr int kNoRow = 1 << 20;
+
+// Most cells of a list that the row count takes: all but two of the board's
+// (TMAX squared for squares, 64 leaves and the sentinel for Lunnon maps).
+template <bool kSym, int TMAX>
+__host__ __device__ constexpr int tail_cells() {
+    return kSym && TMAX > 2 ? TMAX * TMAX - 2 : 63;
+}
+
+template <bool kSym, int TMAX>
+__host__ __device__ constexpr size_t tail_bytes(int tpb) {
+    if constexpr (TMAX > 0) return size_t(tpb / 32) * TailLayout<TMAX, tail_cells<kSym, TMAX>(), kTailFill>::kBytes;
+    else return 0;
+}
+
+template <bool kSym, int TMAX>
+__device__ __forceinline__ uint8_t *tail_of_warp(uint8_t *areas) {
+    return areas + tail_bytes<kSym, TMAX>(int(threadIdx.x) & ~31);
+}
+
+// The pages of the last row of a square: the row's last cell is `last`, held
+// by last - 1 and by a cell of the row before.
+__device__ __forceinline__ TailPages sym_row_pages(const uint8_t *edge, int last) {
+    TailPages r{edge, edge, edge};
+    for (int p = 0; p < 4; ++p) {
+        const uint8_t *e = edge + p * kSymCells;
+        if (e[last] == last - 1) r.a1 = e;
+        else if (e[last] < last) r.b = e;
+        if (e[last - 1] == last - 2) r.a0 = e;
+    }
+    return r;
+}
+
+// Whether the arcs of the placed cells cross on no page: a page of k arcs has
+// k + 1 faces then and only then.  The row count takes that for granted; a
+// unit that a caller made up otherwise is searched by the list walk alone.
+template <class List>
+__device__ __forceinline__ bool pages_planar(const List &L, const uint8_t *edge, int placed) {
+    bool planar = placed <= kSymCells;
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {
+        const uint8_t *e = edge + p * kSymCells;
+        uint64_t left = low_bits(placed);
+        int faces = 0, ends = 0;
+        while (left) {
+            const int g0 = low_bit(left);
+            int g = g0;
+            do {
+                left &= ~(1ULL << g);
+                const int c = L.get(g);
+                const int q = e[c];
+                ends += q < placed;
+                g = q < placed ? q : c;
+            } while (g != g0);
+            ++faces;
+        }
+        planar &= faces == ends / 2 + 1;
+    }
+    return planar;
+}
+
 struct SymSource {
     const uint8_t *cycles;
     int start_i;
     int last;
+    int row;  // cells of the board's last row (0: counted to a partial depth)
 };
 
 struct LunnonSource {
@@ -142,7 +209,11 @@ struct LunnonSource {
 // always safe, because the warp that owns a split item's parent keeps looping
 // until it has nothing left.  The last warp out checks that the work
 // accounting closed (leave_and_check).
-template <int TPB, int WORDS, bool kSym, class Stk>
+//
+// With TMAX > 0 a lane that comes to the last row (of up to TMAX cells) stops
+// there, and once kTailRoots lanes have (or no lane can go on) the warp counts
+// their rows together on masks (tail.cuh).
+template <int TPB, int WORDS, bool kSym, int TMAX, class Stk>
 __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                                                 const LunnonInstanceDev *s_inst,
                                                 const SymSource &sym, const LunnonSource &lun,
@@ -150,7 +221,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                                                 unsigned long long *counts,
                                                 unsigned long long *nodes_out, const Queue &Q,
                                                 uint32_t period, uint32_t wait_limit,
-                                                const List<TPB> &L, Stk &S) {
+                                                const List<TPB> &L, Stk &S, uint8_t *tail_area) {
     constexpr int kVecs = (WORDS + 3) / 4;
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
@@ -168,6 +239,19 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                              reinterpret_cast<const uint32_t *>(s_tables + 4 * kSymCells),
                              s_tables + 8 * kSymCells, sym.start_i};
     LunnonRules lrules{s_tables, 0, 0};
+    using RowTail = Tail<kSym, (TMAX > 0 ? TMAX : 2), tail_cells<kSym, TMAX>(), kTailFill>;
+    RowTail tail;
+    tail.area = tail_area;
+    tail.lane = lane;
+    TailPages pages{};
+    int row_level = kNoRow;  // first level of the last row
+    bool by_walk = false;    // the node at hand has too many gaps for the row count
+    if constexpr (TMAX > 0 && kSym) {
+        if (sym.row > 0) {
+            row_level = sym.last + 1 - sym.row;
+            pages = sym_row_pages(s_tables, sym.last);
+        }
+    }
 
     // Prefetch state: 0 = no initial unit left for this lane, 1 = index
     // taken.  The first indices come from one warp-aggregated atomicAdd.
@@ -199,11 +283,23 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         ++finished;
     };
 
+    int row_len = 0;  // Lunnon: leaves of a row of the map
     auto set_instance = [&](uint32_t inst) -> int {
         const LunnonInstanceDev I = s_inst[inst];
         lrules = LunnonRules{s_tables + I.table_offset, I.n, I.dim};
         last = I.n;
         S.base = I.start_leaf;
+        if constexpr (TMAX > 0) {
+            const int row = I.row < TMAX ? I.row : TMAX;
+            row_level = row >= 2 ? I.n + 1 - row : kNoRow;
+            // Partner tables: neighbour rows of the last two leaves, dimension
+            // 0 along the row, dimension 1 across.
+            const int w = I.n + 1;
+            pages.a1 = lrules.table + I.n * w;
+            pages.a0 = lrules.table + (I.n - 1) * w;
+            pages.b = lrules.table + (w + I.n) * w;
+            row_len = I.row;
+        }
         return I.start_leaf;
     };
 
@@ -227,6 +323,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             if (kSym) {
                 last = sym.last;
                 S.base = sym.start_i;
+                if constexpr (TMAX > 0) row_level = w[21] ? sym.last + 1 - sym.row : kNoRow;
             } else {
                 set_instance(owner);
             }
@@ -265,6 +362,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         w[18] = uint32_t(m);
         w[19] = uint32_t(m >> 32);
         w[20] = uint32_t(s);
+        if (TMAX > 0 && kSym) w[21] = row_level != kNoRow;
         replay_keeping_pick(L, S, s, lvl);
         ring_put(Q, first + rank, w);
     };
@@ -290,6 +388,9 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                     last = sym.last;
                     S.base = root;
                     ok = list_valid(L, root);
+                    if constexpr (TMAX > 0)
+                        row_level = sym.row > 0 && ok && pages_planar(L, s_tables, root)
+                                        ? sym.last + 1 - sym.row : kNoRow;
                 } else {
                     owner = pre_owner;
                     root = set_instance(owner);
@@ -363,7 +464,10 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         nap = 256;
         // One round of evaluation per busy lane: a walk takes at most
         // kWalkCap steps and goes on in the next round if unfinished.
-        if (busy) {
+        auto at_row = [&]() {
+            return TMAX > 0 && busy && eval >= row_level && eval < last && !by_walk;
+        };
+        if (busy && !at_row()) {
             uint64_t g = 0;
             bool evaluated;
             if (kSym) {
@@ -383,12 +487,51 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             }
             if (evaluated) {
                 walking = false;
+                by_walk = false;
                 eval = apply_advance(L, S, lvl, eval, root, last, fresh, g, leaves);
                 fresh = false;
                 if (eval < 0) {
                     flush();
                     busy = false;
                 }
+            }
+        }
+        if constexpr (TMAX > 0) {
+            const bool here = at_row();
+            const unsigned at = __ballot_sync(kFull, here);
+            if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
+                const int K0 = last - eval;
+                uint32_t C = 0, R = 0, H = 0, counted = 0;
+                uint32_t W[RowTail::kRow] = {};
+                bool ok = false;
+                tail.prepare_setup();
+                if (here) {
+                    auto w = [&](int e) -> int {
+                        return kSym ? int(pages.b[last - e]) : last - e - row_len;
+                    };
+                    const int prev = eval > last + 1 - (kSym ? sym.row : row_len) ? eval - 1 : -1;
+                    ok = tail.setup(L, eval, K0, pages, w, prev, C, W, R, H);
+                    if (ok) {
+                        counted = __popc(C) + (kSym ? 1 : 0);
+                        if (!kSym) C &= ~(tail.word(RowTail::Y::kTop)[lane] & 1);
+                    } else {
+                        by_walk = true;
+                    }
+                }
+                tail.enqueue_roots(ok, K0, C, W, R, H);
+                tail.drain(counted);
+                nodes += counted;
+                if (ok) {
+                    leaves += tail.word(RowTail::Y::kAcc)[lane];
+                    eval = apply_advance(L, S, lvl, eval, root, last, fresh, 0, leaves);
+                    fresh = false;
+                    if (eval < 0) {
+                        flush();
+                        busy = false;
+                    }
+                }
+                __syncwarp();
+                round += kTailRounds;
             }
         }
         if (!bookkeeping) continue;
@@ -431,7 +574,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
     }
 }
 
-template <int TPB, int LEVELS>
+template <int TPB, int LEVELS, int TMAX>
 __global__ void __launch_bounds__(TPB)
     sym_batched_kernel(const uint8_t *__restrict__ edges, SymSource src, unsigned long long num,
                        unsigned long long *counts, unsigned long long *nodes_out, Queue Q,
@@ -444,13 +587,14 @@ __global__ void __launch_bounds__(TPB)
     typename StackOf<TPB, LEVELS>::type S;
     init_stack<TPB, 16, LEVELS>(S, smem, tables);
     LunnonSource none{};
-    persistent_loop<TPB, 16, true>(smem, nullptr, src, none, num, counts, nodes_out, Q, period,
-                                   wait_limit, L, S);
+    persistent_loop<TPB, 16, true, TMAX>(smem, nullptr, src, none, num, counts, nodes_out, Q, period,
+                                         wait_limit, L, S,
+                                         tail_of_warp<true, TMAX>(smem + tables + C::kThreadBytes));
 }
 
 // Shared memory: the maps' neighbour tables and their instance records
 // (meta_bytes in all, records at inst_offset), then the carve.
-template <int TPB, int LEVELS>
+template <int TPB, int LEVELS, int TMAX>
 __global__ void __launch_bounds__(TPB)
     lunnon_batched_kernel(const uint8_t *__restrict__ meta, uint32_t meta_bytes,
                           uint32_t inst_offset, LunnonSource src, unsigned long long num,
@@ -465,8 +609,10 @@ __global__ void __launch_bounds__(TPB)
     typename StackOf<TPB, LEVELS>::type S;
     init_stack<TPB, 17, LEVELS>(S, smem, meta_bytes);
     SymSource none{};
-    persistent_loop<TPB, 17, false>(smem, reinterpret_cast<const LunnonInstanceDev *>(smem + inst_offset),
-                                    none, src, num, counts, nodes_out, Q, period, wait_limit, L, S);
+    persistent_loop<TPB, 17, false, TMAX>(
+        smem, reinterpret_cast<const LunnonInstanceDev *>(smem + inst_offset), none, src, num, counts,
+        nodes_out, Q, period, wait_limit, L, S,
+        tail_of_warp<false, TMAX>(smem + meta_bytes + C::kThreadBytes));
 }
 
 // ------------------------------------------------------- launch helpers --
@@ -671,7 +817,7 @@ cudaError_t launch_lunnon_plain(const uint8_t *d_table, int n, int dim, int star
     return cudaGetLastError();
 }
 
-cudaError_t launch_sym_batched(const uint8_t *d_edges, int start_i, int stop_i,
+cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int stop_i,
                                const uint8_t *d_cycles, uint64_t num, uint64_t *d_counts,
                                uint64_t *d_nodes, void *d_workspace, const BatchKnobs &knobs,
                                cudaStream_t stream) {
@@ -679,38 +825,49 @@ cudaError_t launch_sym_batched(const uint8_t *d_edges, int start_i, int stop_i,
     cudaError_t e = cudaMemsetAsync(d_counts, 0, num * sizeof(uint64_t), stream);
     if (e != cudaSuccess) return e;
     const int sms = device_sm_count();
-    const SymSource src{d_cycles, start_i, stop_i - 1};
+    // The row count pays while a unit's search still enters the last row from
+    // above or near its start; a search to a partial depth has no last row.
+    const int row = stop_i == n * n && n >= 5 && start_i <= stop_i - n + 1 ? n : 0;
+    const SymSource src{d_cycles, start_i, stop_i - 1, row};
     const int levels = pick_levels(stop_i - 1 - start_i, knobs.stack_mode == 1);
     const size_t tables = sym_tables_bytes(stop_i - start_i);
     auto *counts = reinterpret_cast<unsigned long long *>(d_counts);
     auto *nodes = reinterpret_cast<unsigned long long *>(d_nodes);
     int bpsm = 0;
-#define MF_SYM_BATCHED(TPB, LV)                                                                  \
+#define MF_SYM_BATCHED(TPB, LV, TM)                                                              \
     do {                                                                                         \
-        const size_t smem = tables + Carve<TPB, 16, LV>::kThreadBytes;                           \
-        e = prepare(sym_batched_kernel<TPB, LV>, smem, TPB, knobs.blocks_per_sm, bpsm);          \
+        const size_t smem = tables + Carve<TPB, 16, LV>::kThreadBytes + tail_bytes<true, TM>(TPB);     \
+        e = prepare(sym_batched_kernel<TPB, LV, TM>, smem, TPB, knobs.blocks_per_sm, bpsm);      \
         if (e != cudaSuccess) return e;                                                          \
         const LaunchShape shape =                                                                \
             persistent_shape(sms, bpsm, TPB, num, stop_i - start_i, knobs.queue_capacity);       \
         const Queue Q = carve_queue(d_workspace, shape.ring);                                    \
         e = reset_queue(Q, stream);                                                              \
         if (e != cudaSuccess) return e;                                                          \
-        sym_batched_kernel<TPB, LV><<<shape.blocks, TPB, smem, stream>>>(                        \
+        sym_batched_kernel<TPB, LV, TM><<<shape.blocks, TPB, smem, stream>>>(                    \
             d_edges, src, num, counts, nodes, Q, knobs.node_budget, knobs.wait_limit);          \
     } while (0)
-    if (knobs.block_threads == 256) {
+    if (row == 8) {
+        MF_SYM_BATCHED(128, 0, 8);
+    } else if (row == 7) {
+        MF_SYM_BATCHED(128, 0, 7);
+    } else if (row == 6) {
+        MF_SYM_BATCHED(128, 0, 6);
+    } else if (row == 5) {
+        MF_SYM_BATCHED(128, 0, 5);
+    } else if (knobs.block_threads == 256) {
         switch (levels) {
-            case 24: MF_SYM_BATCHED(256, 24); break;
-            case 32: MF_SYM_BATCHED(256, 32); break;
-            case 48: MF_SYM_BATCHED(256, 48); break;
-            default: MF_SYM_BATCHED(256, 0); break;
+            case 24: MF_SYM_BATCHED(256, 24, 0); break;
+            case 32: MF_SYM_BATCHED(256, 32, 0); break;
+            case 48: MF_SYM_BATCHED(256, 48, 0); break;
+            default: MF_SYM_BATCHED(256, 0, 0); break;
         }
     } else {
         switch (levels) {
-            case 24: MF_SYM_BATCHED(128, 24); break;
-            case 32: MF_SYM_BATCHED(128, 32); break;
-            case 48: MF_SYM_BATCHED(128, 48); break;
-            default: MF_SYM_BATCHED(128, 0); break;
+            case 24: MF_SYM_BATCHED(128, 24, 0); break;
+            case 32: MF_SYM_BATCHED(128, 32, 0); break;
+            case 48: MF_SYM_BATCHED(128, 48, 0); break;
+            default: MF_SYM_BATCHED(128, 0, 0); break;
         }
     }
 #undef MF_SYM_BATCHED
@@ -732,33 +889,33 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
     auto *counts = reinterpret_cast<unsigned long long *>(d_counts);
     auto *nodes = reinterpret_cast<unsigned long long *>(d_nodes);
     int bpsm = 0;
-#define MF_LUN_BATCHED(TPB, LV)                                                                  \
+#define MF_LUN_BATCHED(TPB, LV, TM)                                                              \
     do {                                                                                         \
-        const size_t smem = mb + Carve<TPB, 17, LV>::kThreadBytes;                               \
-        e = prepare(lunnon_batched_kernel<TPB, LV>, smem, TPB, knobs.blocks_per_sm, bpsm);       \
+        const size_t smem = mb + Carve<TPB, 17, LV>::kThreadBytes + tail_bytes<false, TM>(TPB);         \
+        e = prepare(lunnon_batched_kernel<TPB, LV, TM>, smem, TPB, knobs.blocks_per_sm, bpsm);   \
         if (e != cudaSuccess) return e;                                                          \
         const LaunchShape shape =                                                                \
             persistent_shape(sms, bpsm, TPB, num, max_levels, knobs.queue_capacity);             \
         const Queue Q = carve_queue(d_workspace, shape.ring);                                    \
         e = reset_queue(Q, stream);                                                              \
         if (e != cudaSuccess) return e;                                                          \
-        lunnon_batched_kernel<TPB, LV><<<shape.blocks, TPB, smem, stream>>>(                     \
+        lunnon_batched_kernel<TPB, LV, TM><<<shape.blocks, TPB, smem, stream>>>(                 \
             d_meta, mb, inst_offset, src, num, counts, nodes, Q, knobs.node_budget,             \
             knobs.wait_limit);                                                                   \
     } while (0)
     if (knobs.block_threads == 256) {
         switch (levels) {
-            case 24: MF_LUN_BATCHED(256, 24); break;
-            case 32: MF_LUN_BATCHED(256, 32); break;
-            case 48: MF_LUN_BATCHED(256, 48); break;
-            default: MF_LUN_BATCHED(256, 0); break;
+            case 24: MF_LUN_BATCHED(256, 24, 0); break;
+            case 32: MF_LUN_BATCHED(256, 32, 0); break;
+            case 48: MF_LUN_BATCHED(256, 48, 0); break;
+            default: MF_LUN_BATCHED(256, 0, 0); break;
         }
     } else {
         switch (levels) {
-            case 24: MF_LUN_BATCHED(128, 24); break;
-            case 32: MF_LUN_BATCHED(128, 32); break;
-            case 48: MF_LUN_BATCHED(128, 48); break;
-            default: MF_LUN_BATCHED(128, 0); break;
+            case 24: MF_LUN_BATCHED(128, 24, 0); break;
+            case 32: MF_LUN_BATCHED(128, 32, 0); break;
+            case 48: MF_LUN_BATCHED(128, 48, 0); break;
+            default: MF_LUN_BATCHED(128, 0, 0); break;
         }
     }
 #undef MF_LUN_BATCHED
@@ -900,7 +1057,7 @@ extern "C" int32_t mf_sym_count_cases_batched_static(int32_t n, int32_t start_i,
     if (int rc = current_static_state(s)) return rc;
     BatchKnobs knobs = resolve_knobs(cfg);
     knobs.queue_capacity = kStaticRingCells;
-    MF_TRY_CUDA(launch_sym_batched(s->edges + size_t(n) * 4 * kSymCells, start_i, stop_i, d_cycles,
+    MF_TRY_CUDA(launch_sym_batched(s->edges + size_t(n) * 4 * kSymCells, n, start_i, stop_i, d_cycles,
                                    num_cases, d_counts, d_nodes, s->workspace, knobs,
                                    static_cast<cudaStream_t>(stream)));
     return MF_OK;

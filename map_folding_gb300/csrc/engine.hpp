@@ -193,6 +193,7 @@ struct LunnonInstanceDev {
     int32_t n;
     int32_t dim;
     int32_t start_leaf;
+    int32_t row;  // leaves of the last row of a 2-D map (0: no such row)
 };
 
 // d_edges: the 4 x 64 edge pages in device memory.
@@ -209,7 +210,7 @@ cudaError_t launch_sym_wide(const uint8_t *d_wide_edges, int start_i, int stop_i
                             uint64_t *d_nodes, void *d_workspace, const BatchKnobs &knobs,
                             cudaStream_t stream);
 
-cudaError_t launch_sym_batched(const uint8_t *d_edges, int start_i, int stop_i,
+cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int stop_i,
                                const uint8_t *d_cycles, uint64_t num, uint64_t *d_counts,
                                uint64_t *d_nodes, void *d_workspace, const BatchKnobs &knobs,
                                cudaStream_t stream);

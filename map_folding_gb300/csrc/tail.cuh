@@ -1,0 +1,419 @@
+// tail.cuh -- the last row of the search, counted on 32-bit masks.
+//
+// On both paths the last cells to be placed form a row v_0 .. v_{T-1} of the
+// board (the spiral's last side; the last row of a 2-D Lunnon map), and 96 %
+// of a 7x7 search's nodes lie there.  Each row cell v_t is held by two arcs:
+// one to w_t, its neighbour in the row before, on one page b for the whole
+// row, and one to v_{t-1}, on two pages that alternate along the row.  So
+// instead of inserting the row's cells into the list and walking both pages
+// again at every node, a warp takes 32 "roots" (lists that end where the row
+// begins), writes down once per root what the row can see of the list, and
+// counts every completion on masks:
+//
+//   U        the gaps of the list that are in the page-b face of some pending
+//            w_x: no row cell can ever go anywhere else.  At most 31 of them
+//            (17 on average on 7x7 and 8x8); numbered in list order, so a set
+//            of gaps is a 32-bit mask and "after" is "greater".
+//   W[x]     the face of w_x on page b: where v_x may still go.
+//   P[x]     the gaps before w_x in list order (ones below a bit).
+//   planes   the faces of the gaps on the two row pages, as five bit planes of
+//            face numbers each: the gaps in the face of gap r are those whose
+//            plane bits equal r's.
+//
+// Placing v_t into gap r (bit b) draws the arc (w_t, v_t) on page b; every
+// pending face is on one side of it, W[x] &= that side, where gap r itself,
+// if W[x] has it, is cut in two and W[x] keeps the half on its side.  Which
+// half is one bit h(x, t): every pending W[x] holds at most one piece of each
+// gap, so base gaps stay exact positions.  The gaps that the next cell may
+// take are r's row-page face & W[x], cut by the row arcs drawn earlier on the same
+// page: v_t and v_{t+1} lie on the same side of each.  With A(s, x) = the
+// gaps whose piece seen by x is after v_s = h ? -b_s : -2 b_s, an arc (v_s,
+// v_{s+1}) encloses A(s, x) ^ A(s+1, x).
+//
+// The levels are counted from the end: e = T-1-t, so v at level K has K row
+// cells after it.  A frame (candidates C of level K, W[K-1..0], the earlier
+// picks, the h bits) is one partly counted node.  All lanes of a warp step
+// through the levels together: at each level, idle lanes take a frame from
+// the level's queue, every lane places its frame's next candidate, and what
+// is left of the frame goes back to the queue.  A frame may run on any lane;
+// leaves are added up per root slot.
+#pragma once
+
+#include "dfs_core.cuh"
+
+namespace mf {
+namespace {
+
+// What a warp keeps in shared memory for its rows.  CELLS: the most cells a
+// root's list can have.  A level with FILL or more frames is run before a
+// shallower one, so no level ever holds more than FILL - 1 + 32.
+template <int TMAX, int CELLS, int FILL>
+struct TailLayout {
+    static_assert(CELLS <= 63 && FILL <= 32 && TMAX >= 2 && TMAX <= 8, "tail layout");
+    static constexpr int kCap = FILL + 32;
+    __host__ __device__ static constexpr int quads(int k) { return (3 + k + 3) / 4; }
+    __host__ __device__ static constexpr int cap(int k) { return k == TMAX - 1 ? 32 : kCap; }
+    __host__ __device__ static constexpr int frames(int k) {  // offset of level k's queue
+        int at = kFrames;
+        for (int j = 1; j < k; ++j) at += quads(j) * cap(j) * 16;
+        return at;
+    }
+    static constexpr int kPlane = 0;                         // 2 pages x 5 planes
+    static constexpr int kBefore = kPlane + 10 * 128;        // P of each level
+    static constexpr int kTop = kBefore + TMAX * 128;        // Lunnon: bit 0 the gap on the sentinel,
+                                                             // << 8 the first level with an arc
+    static constexpr int kAcc = kTop + 128;                  // leaves of each root
+    static constexpr int kFrames = kAcc + 128;
+    // Scratch of the set-up, in the frames' place (they are empty then): per
+    // cell the face numbers before it and its place in the list, per place the
+    // face numbers after it; then the same of U's gaps only.
+    static constexpr int kPre = kFrames;
+    static constexpr int kIds = kPre + ((CELLS + 1) / 2 * 2) * 64;
+    static constexpr int kPos = kIds + CELLS * 64;
+    static constexpr int kScratchEnd = kPos + CELLS * 32;
+    static constexpr int kGapIds = kPre;
+    static_assert(kPre + 16 * 128 <= kIds || CELLS < 32, "gap ids lie over the cells' face numbers");
+    static constexpr int kEnd = frames(TMAX);
+    static constexpr int kBytes = ((kEnd > kScratchEnd ? kEnd : kScratchEnd) + 127) / 128 * 128;
+};
+
+// 1 << k, 0 for k >= 32.
+__device__ __forceinline__ uint32_t bit32(uint32_t k) {
+    uint32_t r;
+    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(1u), "r"(k));
+    return r;
+}
+
+// The row's pages: partner tables of the placed cells (an entry >= the
+// number of placed cells: none).
+struct TailPages {
+    const uint8_t *b;   // page of the arcs (w_t, v_t)
+    const uint8_t *a0;  // page of the arc from a cell of an even level
+    const uint8_t *a1;  // ... of an odd level
+};
+
+// kSym: a square's side, always of TMAX cells; else rows of a Lunnon map, of up
+// to TMAX leaves (a longer row starts inside), whose gap on the sentinel counts
+// as a node and is not searched.
+template <bool kSym, int TMAX, int CELLS, int FILL>
+struct Tail {
+    using Y = TailLayout<TMAX, CELLS, FILL>;
+    static constexpr int kRow = TMAX;
+    uint8_t *area;
+    int lane;
+    int cnt[TMAX];  // frames queued per level 1 .. TMAX-1 (warp-uniform)
+
+    __device__ __forceinline__ uint32_t *word(int off) const {
+        return reinterpret_cast<uint32_t *>(area + off);
+    }
+    // Bit of h(ex, es): the half of v_es's gap that the pending level ex keeps.
+    __device__ static constexpr int hbit(int ex, int es) { return es * (es - 1) / 2 - 1 + ex; }
+
+    // Clear the set-up's scratch for lists of `placed` cells (all lanes call).
+    __device__ __forceinline__ void prepare_setup() const {
+        uint4 *pre = reinterpret_cast<uint4 *>(area + Y::kPre);
+#pragma unroll
+        for (int k = 0; k < (Y::kIds - Y::kPre) / 16; k += 32)
+            if (k + lane < (Y::kIds - Y::kPre) / 16) pre[k + lane] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        __syncwarp();
+    }
+
+    // Write down a root: the list L of `placed` cells, row levels K0 .. 0 to
+    // come, w(e) the row-before neighbour of level e's cell and prev the cell
+    // before the first (< 0: none, the row starts here).  Returns false if it
+    // has more than 31 gaps.  Fills the root's tables and hands back the frame
+    // in registers.
+    //
+    // One pass over the list in order, with no data-dependent branch so that
+    // all lanes stay together: going past the first end of an arc enters a new
+    // face, past the second end returns to the face before the first.  (Walking
+    // each face by itself took 8 times as long, the lanes' walks being of
+    // different lengths.)  The face numbers of the gaps in U, one 16-bit word
+    // per gap, are then turned into planes by a 16 x 16 bit transposition.
+    template <class List, class WOf>
+    __device__ __forceinline__ bool setup(const List &L, int placed, int K0, const TailPages &pg,
+                                          WOf &&w, int prev, uint32_t &C, uint32_t (&W)[TMAX],
+                                          uint32_t &R, uint32_t &H) const {
+        uint16_t *pre = reinterpret_cast<uint16_t *>(area + Y::kPre) + lane;
+        uint16_t *ids = reinterpret_cast<uint16_t *>(area + Y::kIds) + lane;
+        uint8_t *pos = area + Y::kPos + lane;
+        // Face numbers of the gap at hand and the highest given out: page b in
+        // bits 0-4, a0 in 5-9, a1 in 10-14.
+        uint32_t f = 0, top = 0;
+        int c = 0;
+#pragma unroll 1
+        for (int i = 0; i < placed; ++i) {
+            pre[c * 32] = uint16_t(f);
+            pos[c * 32] = uint8_t(i);
+            const int after = L.get(c);
+            const int q0 = pg.b[c], q1 = pg.a0[c], q2 = pg.a1[c];
+            // No placed partner: c's own entry, which changes nothing.
+            const uint32_t v0 = pre[(q0 < placed ? q0 : c) * 32];
+            const uint32_t v1 = pre[(q1 < placed ? q1 : c) * 32];
+            const uint32_t v2 = pre[(q2 < placed ? q2 : c) * 32];
+            if (v0 == 0xffffu) top += 1u;
+            if (v1 == 0xffffu) top += 1u << 5;
+            if (v2 == 0xffffu) top += 1u << 10;
+            f = ((v0 == 0xffffu ? top : v0) & 0x001fu) | ((v1 == 0xffffu ? top : v1) & 0x03e0u) |
+                ((v2 == 0xffffu ? top : v2) & 0x7c00u);
+            ids[i * 32] = uint16_t(f);
+            c = after;
+        }
+        // Not one cycle (cell 0 met again before the end): left to the list walk.
+        if (c != 0 || pos[0] != 0) return false;
+        // The faces of the w's on page b (a w has no arc there, so its gap is
+        // in the face before it).
+        uint32_t fw[TMAX];
+        int at[TMAX];
+        uint32_t set = 0;
+#pragma unroll
+        for (int e = 0; e < TMAX; ++e) {
+            fw[e] = 0;
+            at[e] = 0;
+            if (e <= K0) {
+                const int x = w(e);
+                fw[e] = pre[x * 32] & 31u;
+                at[e] = pos[x * 32];
+                set |= 1u << fw[e];
+            }
+        }
+        const uint32_t fprev = prev >= 0 ? pre[prev * 32] : 0;
+        // U in list order.
+        uint64_t places = 0;
+        int gaps = 0;
+        uint16_t *gap_ids = reinterpret_cast<uint16_t *>(area + Y::kGapIds) + 2 * lane;
+#pragma unroll 2
+        for (int i = 0; i < placed; ++i) {
+            const uint32_t v = ids[i * 32];
+            const bool in = (set >> (v & 31)) & 1;
+            if (in && gaps < 32) {
+                gap_ids[(gaps & 15) * 64 + (gaps >> 4)] = uint16_t(v);
+                places |= 1ULL << i;
+            }
+            gaps += in;
+        }
+        if (gaps > 31) return false;
+        uint32_t a[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) a[j] = word(Y::kGapIds)[j * 32 + lane];
+#pragma unroll
+        for (int t = 8; t >= 1; t >>= 1) {
+            const uint32_t m = t == 8 ? 0x00ff00ffu : t == 4 ? 0x0f0f0f0fu
+                               : t == 2 ? 0x33333333u : 0x55555555u;
+#pragma unroll
+            for (int j = 0; j < 16; ++j)
+                if (!(j & t)) {
+                    const uint32_t x = ((a[j] >> t) ^ a[j + t]) & m;
+                    a[j + t] ^= x;
+                    a[j] ^= x << t;
+                }
+        }
+#pragma unroll
+        for (int j = 0; j < 10; ++j) word(Y::kPlane)[j * 32 + lane] = a[5 + j];
+        const uint32_t all = (1u << gaps) - 1;
+        C = 0;
+#pragma unroll
+        for (int e = TMAX - 1; e >= 0; --e) {
+            uint32_t m = all;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) m &= (fw[e] >> j) & 1 ? a[j] : ~a[j];
+            W[e] = e <= K0 ? m : 0;
+            if (e == K0) C = m;
+            word(Y::kBefore)[e * 32 + lane] = (1u << __popcll(places & low_bits(at[e]))) - 1;
+        }
+        if (!kSym)
+            word(Y::kTop)[lane] = uint32_t(places & 1) | uint32_t(prev >= 0 ? TMAX : K0) << 8;
+        R = 0;
+        H = uint32_t(lane) << 27;
+        if (prev >= 0) {
+            // v_{t-1} is a cell of the list: its face on the page of the next
+            // arc, and it stands in for all earlier picks (an arc between two
+            // equal picks encloses nothing).
+            const bool odd = (K0 + 1) & 1;
+            const uint32_t fp = odd ? fprev >> 10 : fprev >> 5;
+            uint32_t m = ~0u;
+#pragma unroll
+            for (int j = 0; j < 5; ++j) {
+                const uint32_t plane = word(Y::kPlane)[((odd ? 5 : 0) + j) * 32 + lane];
+                m &= (fp >> j) & 1 ? plane : ~plane;
+            }
+            C &= m;
+            const uint32_t before = uint32_t(__popcll(places & low_bits(pos[prev * 32])));
+#pragma unroll
+            for (int j = 0; j < 6; ++j) R |= before << (5 * j);
+            H |= (~0u << hbit(0, K0 + 1)) & 0x07ffffffu;
+        }
+        return true;
+    }
+
+    // Put the root frames of the lanes in `have` into their levels' queues
+    // (all lanes call; the set-up's scratch is given up here).
+    __device__ __forceinline__ void enqueue_roots(bool have, int K0, uint32_t C, uint32_t (&W)[TMAX],
+                                                  uint32_t R, uint32_t H) {
+        word(Y::kAcc)[lane] = 0;
+        __syncwarp();
+        push_roots<TMAX - 1>(have, K0, C, W, R, H);
+        __syncwarp();
+    }
+
+    template <int K>
+    __device__ __forceinline__ void push_roots(bool have, int K0, uint32_t C, uint32_t (&W)[TMAX],
+                                               uint32_t R, uint32_t H) {
+        if constexpr (K >= 1) {
+            cnt[K] = 0;
+            push<K>(have && K0 == K && C != 0, C, W, R, H);
+            push_roots<K - 1>(have, K0, C, W, R, H);
+        }
+    }
+
+    template <int K>
+    __device__ __forceinline__ void push(bool mine, uint32_t C, const uint32_t (&W)[TMAX], uint32_t R,
+                                         uint32_t H) {
+        const unsigned m = __ballot_sync(kFull, mine);
+        if (!m) return;
+        const int at = cnt[K] + __popc(m & ((1u << lane) - 1));
+        cnt[K] += __popc(m);
+        if (mine) {
+            uint32_t w[4 * Y::quads(K)] = {};
+            w[0] = C;
+            w[1] = R;
+            w[2] = H;
+#pragma unroll
+            for (int e = 0; e < K; ++e) w[3 + e] = W[e];
+            uint4 *q = reinterpret_cast<uint4 *>(area + Y::frames(K)) + at;
+#pragma unroll
+            for (int j = 0; j < Y::quads(K); ++j)
+                q[j * Y::cap(K)] = make_uint4(w[4 * j], w[4 * j + 1], w[4 * j + 2], w[4 * j + 3]);
+        }
+    }
+
+    // Idle lanes (C == 0) take frames of level K.
+    template <int K>
+    __device__ __forceinline__ void refill(uint32_t &C, uint32_t (&W)[TMAX], uint32_t (&b)[TMAX],
+                                           uint32_t &R, uint32_t &H) {
+        const unsigned idle = __ballot_sync(kFull, C == 0);
+        const int want = __popc(idle);
+        const int take = want < cnt[K] ? want : cnt[K];
+        const int rank = __popc(idle & ((1u << lane) - 1));
+        cnt[K] -= take;
+        if (C == 0 && rank < take) {
+            const uint4 *q = reinterpret_cast<const uint4 *>(area + Y::frames(K)) + cnt[K] + rank;
+            uint32_t w[4 * Y::quads(K)];
+#pragma unroll
+            for (int j = 0; j < Y::quads(K); ++j) {
+                const uint4 x = q[j * Y::cap(K)];
+                w[4 * j] = x.x;
+                w[4 * j + 1] = x.y;
+                w[4 * j + 2] = x.z;
+                w[4 * j + 3] = x.w;
+            }
+            C = w[0];
+            R = w[1];
+            H = w[2];
+#pragma unroll
+            for (int e = 0; e < K; ++e) W[e] = w[3 + e];
+#pragma unroll
+            for (int e = K + 1; e < TMAX; ++e) b[e] = 1u << ((R >> (5 * (e - K - 1))) & 31);
+        }
+        __syncwarp();
+    }
+
+    // A(es, ex): the gaps whose piece seen by level ex is after v_es.
+    __device__ static __forceinline__ uint32_t after(const uint32_t (&b)[TMAX], uint32_t H, int ex,
+                                                     int es) {
+        const uint32_t n = 0u - b[es];
+        return (H >> hbit(ex, es)) & 1 ? n : n + n;
+    }
+
+    // Level K of a descent: idle lanes take frames, every lane takes its
+    // frame's next candidate and queues the rest (twice, so that lanes still
+    // idle share the candidates of frames just taken: 28 of 32 lanes busy
+    // instead of 20 on 7x7 roots); then the candidates are placed, and the
+    // placed cells' frames go on to the next level.
+    template <int K>
+    __device__ __forceinline__ void levels(int start, uint32_t &C, uint32_t (&W)[TMAX],
+                                           uint32_t (&b)[TMAX], uint32_t &R, uint32_t &H,
+                                           uint32_t &nodes) {
+        if constexpr (K >= 1) {
+            if (K <= start) {
+                uint32_t bt = 0;
+#pragma unroll 1
+                for (int turn = 0; turn < 2; ++turn) {
+                    if (cnt[K] > 0) refill<K>(C, W, b, R, H);
+                    const uint32_t rest = bt ? 0 : C & (C - 1);
+                    if (!bt) bt = C & (0u - C);
+                    push<K>(rest != 0, rest, W, R, H);
+                    __syncwarp();
+                    if (cnt[K] == 0 || __all_sync(kFull, bt != 0)) break;
+                }
+                uint32_t next = 0;
+                if (bt) {
+                    const int slot = int(H >> 27);
+                    const uint32_t info = kSym ? 0 : word(Y::kTop)[slot];
+                    const int r = 31 - __clz(int(bt));
+                    const uint32_t *before = word(Y::kBefore) + slot;
+                    const uint32_t *plane = word(Y::kPlane) + (K & 1) * 160 + slot;
+                    uint32_t face = ~0u;
+#pragma unroll
+                    for (int j = 0; j < 5; ++j) {
+                        const uint32_t p = plane[j * 32];
+                        face &= p & bt ? p : ~p;
+                    }
+                    const uint32_t pt = before[K * 32];
+                    const uint32_t side = pt ^ (bt - 1);
+                    const uint32_t inside = side | bt, outside = ~side | bt;
+                    const bool up = bt > pt;
+#pragma unroll
+                    for (int e = K - 1; e >= 0; --e) {
+                        const uint32_t pe = before[e * 32];
+                        const bool in = (pe >= bt) != (pe > pt);
+                        W[e] &= in ? inside : outside;
+                        if constexpr (K >= 2)
+                            if (in != up) H |= 1u << hbit(e, K);
+                    }
+                    next = face & W[K - 1];
+#pragma unroll
+                    for (int es = K + 2; es < TMAX; es += 2) {
+                        const bool enclosed =
+                            ((after(b, H, K, es) ^ after(b, H, K, es - 1)) & bt) != 0;
+                        const uint32_t D = after(b, H, K - 1, es) ^ after(b, H, K - 1, es - 1);
+                        const uint32_t side_of = enclosed ? D : ~D;
+                        // A Lunnon row may be shorter than TMAX: no arc leads
+                        // to its first cell.
+                        next &= kSym || es <= int(info >> 8) ? side_of : ~0u;
+                    }
+                    if (K >= 2 || !kSym) nodes += __popc(next);
+                    next &= ~(info & 1);
+                    if (K == 1) {
+                        if (next) atomicAdd(word(Y::kAcc) + slot, uint32_t(__popc(next)));
+                        next = 0;
+                    }
+                    b[K] = bt;
+                    R = (R << 5) | uint32_t(r);
+                }
+                C = next;
+            }
+            levels<K - 1>(start, C, W, b, R, H, nodes);
+        }
+    }
+
+    // Count the queued frames to the end.
+    __device__ __forceinline__ void drain(uint32_t &nodes) {
+        for (;;) {
+            int start = 0;
+#pragma unroll
+            for (int k = 1; k < TMAX; ++k)
+                if (cnt[k] > 0) start = k;  // the shallowest level with frames ...
+#pragma unroll
+            for (int k = TMAX - 1; k >= 1; --k)
+                if (cnt[k] >= FILL) start = k;  // ... or the deepest full one
+            if (start == 0) return;
+            uint32_t C = 0, R = 0, H = 0;
+            uint32_t W[TMAX] = {}, b[TMAX] = {};
+            levels<TMAX - 1>(start, C, W, b, R, H, nodes);
+        }
+    }
+};
+
+}  // namespace
+}  // namespace mf
