@@ -251,9 +251,10 @@ int32_t mf_lunnon_collect(const mf_lunnon_plan *plan, int32_t depth, uint8_t *st
     return MF_OK;
 }
 
-// Leaves of the last row of a 2-D map with at least two rows (0: no such row).
+// Leaves of the last row of a 2-D map of at least two rows, where that row is
+// counted on masks (0: it is not).  A row of two is one arc and not worth it.
 static int32_t last_row(const LunnonTables &t) {
-    return t.dim == 2 && t.p[0] >= 2 && t.p[1] >= 2 ? t.p[0] : 0;
+    return t.dim == 2 && t.p[0] >= 3 && t.p[1] >= 2 && t.n <= kRowLeaves ? t.p[0] : 0;
 }
 
 static int upload_table(mf_lunnon_plan *plan) {
@@ -455,11 +456,14 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
     MF_TRY_CUDA(cudaMemsetAsync(d_counts + num_plans, 0, 8, st));
     cudaEventRecord(th.b, st);
     cudaEventRecord(tk.a, st);
-    int max_levels = 0;
-    for (const auto &I : inst) max_levels = std::max(max_levels, I.n - I.start_leaf);
+    int max_levels = 0, row_levels = 0;
+    for (const auto &I : inst) {
+        max_levels = std::max(max_levels, I.n - I.start_leaf);
+        if (I.row) row_levels = std::max(row_levels, I.n - I.start_leaf);
+    }
     const uint32_t meta_used = uint32_t(tables.size() + inst.size() * sizeof(LunnonInstanceDev));
     MF_TRY_CUDA(launch_lunnon_batched(d_meta, meta_used, uint32_t(tables.size()), num_plans,
-                                      max_levels, d_units,
+                                      max_levels, row_levels, d_units,
                                       reinterpret_cast<uint32_t *>(d_units + unit_bytes), total,
                                       d_counts, d_counts + num_plans, d_work, knobs, st));
     cudaEventRecord(tk.b, st);
@@ -649,7 +653,7 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
     std::vector<uint8_t> meta;
     std::vector<uint64_t> per_plan(num_plans);
     uint64_t total = 0;
-    int max_levels = 0;
+    int max_levels = 0, row_levels = 0;
     for (int k = 0; k < num_plans; ++k) {
         const mf_lunnon_plan *p = plans[k];
         if (!p) {
@@ -665,6 +669,7 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
         per_plan[k] = collect_lunnon_states(p->t, d, nullptr, 0, stride);
         total += per_plan[k];
         max_levels = std::max(max_levels, p->t.n - d - 1);
+        if (inst[k].row) row_levels = std::max(row_levels, p->t.n - d - 1);
     }
     if (meta.size() > 160 * 1024) {
         set_error("batched maps' tables total %zu bytes; at most 163840 fit on chip", meta.size());
@@ -703,7 +708,7 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
             cudaError_t e = cudaMemsetAsync(raw->d_counts + num_plans, 0, sizeof(uint64_t), s);
             if (e != cudaSuccess) return e;
             return launch_lunnon_batched(raw->d_meta, uint32_t(meta.size()), inst_offset, num_plans,
-                                         max_levels, raw->d_units,
+                                         max_levels, row_levels, raw->d_units,
                                          reinterpret_cast<uint32_t *>(raw->d_units + unit_bytes),
                                          total, raw->d_counts, raw->d_counts + num_plans,
                                          raw->d_work, knobs, s);

@@ -120,12 +120,13 @@ constexpr int kTailFill = 16;    // frames that make a level full
 constexpr int kTailRoots = 28;   // lanes at the row that start a count
 constexpr uint32_t kTailRounds = 8;  // bookkeeping rounds that a count stands for
 constexpr int kNoRow = 1 << 20;
+constexpr int kRowLevels = 4;  // Lunnon: levels to go, of a map with rows, from which they pay
 
-// Most cells of a list that the row count takes: all but two of the board's
-// (TMAX squared for squares, 64 leaves and the sentinel for Lunnon maps).
+// Most cells of a list that the row count takes: all but two of a square's;
+// for Lunnon maps kRowLeaves' worth (what the frames' place holds as scratch).
 template <bool kSym, int TMAX>
 __host__ __device__ constexpr int tail_cells() {
-    return kSym && TMAX > 2 ? TMAX * TMAX - 2 : 63;
+    return kSym && TMAX > 2 ? TMAX * TMAX - 2 : kRowLeaves - 1;
 }
 
 template <bool kSym, int TMAX>
@@ -510,7 +511,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                         return kSym ? int(pages.b[last - e]) : last - e - row_len;
                     };
                     const int prev = eval > last + 1 - (kSym ? sym.row : row_len) ? eval - 1 : -1;
-                    ok = tail.setup(L, eval, K0, pages, w, prev, C, W, R, H);
+                    ok = tail.setup(at, L, eval, K0, pages, w, prev, C, W, R, H);
                     if (ok) {
                         counted = __popc(C) + (kSym ? 1 : 0);
                         if (!kSym) C &= ~(tail.word(RowTail::Y::kTop)[lane] & 1);
@@ -875,10 +876,10 @@ cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int s
 }
 
 cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, uint32_t inst_offset,
-                                  int num_inst, int max_levels, const uint8_t *d_states,
-                                  const uint32_t *d_state_owner, uint64_t num, uint64_t *d_counts,
-                                  uint64_t *d_nodes, void *d_workspace, const BatchKnobs &knobs,
-                                  cudaStream_t stream) {
+                                  int num_inst, int max_levels, int row_levels,
+                                  const uint8_t *d_states, const uint32_t *d_state_owner,
+                                  uint64_t num, uint64_t *d_counts, uint64_t *d_nodes,
+                                  void *d_workspace, const BatchKnobs &knobs, cudaStream_t stream) {
     cudaError_t e = cudaMemsetAsync(d_counts, 0, size_t(num_inst) * sizeof(uint64_t), stream);
     if (e != cudaSuccess) return e;
     if (num == 0) return reset_queue(carve_queue(d_workspace, knobs.queue_capacity), stream);
@@ -903,7 +904,16 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
             d_meta, mb, inst_offset, src, num, counts, nodes, Q, knobs.node_budget,             \
             knobs.wait_limit);                                                                   \
     } while (0)
-    if (knobs.block_threads == 256) {
+    if (row_levels >= kRowLevels) {
+        // All the maps' tables are in every CTA's shared memory, so many small
+        // maps leave room for few CTAs: take the CTA size that keeps more
+        // warps on an SM.
+        const size_t warp = tail_bytes<false, 6>(32) + Carve<32, 17, 0>::kThreadBytes;
+        const size_t room = 227 * 1024;
+        const size_t small = room / (mb + 4 * warp + 1024) * 4;
+        if (mb + 16 * warp <= room && small < 16) MF_LUN_BATCHED(512, 0, 6);
+        else MF_LUN_BATCHED(128, 0, 6);
+    } else if (knobs.block_threads == 256) {
         switch (levels) {
             case 24: MF_LUN_BATCHED(256, 24, 0); break;
             case 32: MF_LUN_BATCHED(256, 32, 0); break;

@@ -187,6 +187,9 @@ int check_queue_header(const QueueHeader &hdr, uint64_t units);
 uint64_t workspace_bytes(uint64_t capacity);
 uint64_t wide_workspace_bytes(uint64_t capacity);
 
+// Largest Lunnon map whose last row is counted on masks.
+constexpr int kRowLeaves = 41;
+
 // One Lunnon map as the batched kernel sees it.
 struct LunnonInstanceDev {
     uint32_t table_offset;  // into the concatenated next-tables
@@ -222,12 +225,13 @@ cudaError_t launch_lunnon_plain(const uint8_t *d_table, int n, int dim, int star
 // d_state_owner[k] = instance of state k; d_counts[instance] += count/leaf.
 // d_meta holds the maps' neighbour tables followed, at inst_offset, by their
 // LunnonInstanceDev records (meta_bytes in all); max_levels is the largest
-// n - start_leaf over the instances.
+// n - start_leaf over the instances, row_levels the largest over those whose
+// last row is counted by itself (row > 0).
 cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, uint32_t inst_offset,
-                                  int num_inst, int max_levels, const uint8_t *d_states,
-                                  const uint32_t *d_state_owner, uint64_t num, uint64_t *d_counts,
-                                  uint64_t *d_nodes, void *d_workspace, const BatchKnobs &knobs,
-                                  cudaStream_t stream);
+                                  int num_inst, int max_levels, int row_levels,
+                                  const uint8_t *d_states, const uint32_t *d_state_owner,
+                                  uint64_t num, uint64_t *d_counts, uint64_t *d_nodes,
+                                  void *d_workspace, const BatchKnobs &knobs, cudaStream_t stream);
 
 int device_sm_count();
 

@@ -68,11 +68,10 @@ struct TailLayout {
     // cell the face numbers before it and its place in the list, per place the
     // face numbers after it; then the same of U's gaps only.
     static constexpr int kPre = kFrames;
-    static constexpr int kIds = kPre + ((CELLS + 1) / 2 * 2) * 64;
+    static constexpr int kIds = kPre + (CELLS > 32 ? (CELLS + 1) / 2 * 2 : 32) * 64;
     static constexpr int kPos = kIds + CELLS * 64;
     static constexpr int kScratchEnd = kPos + CELLS * 32;
-    static constexpr int kGapIds = kPre;
-    static_assert(kPre + 16 * 128 <= kIds || CELLS < 32, "gap ids lie over the cells' face numbers");
+    static constexpr int kGapIds = kPre;  // over the cells' face numbers: 16 words a lane
     static constexpr int kEnd = frames(TMAX);
     static constexpr int kBytes = ((kEnd > kScratchEnd ? kEnd : kScratchEnd) + 127) / 128 * 128;
 };
@@ -120,8 +119,8 @@ struct Tail {
 
     // Write down a root: the list L of `placed` cells, row levels K0 .. 0 to
     // come, w(e) the row-before neighbour of level e's cell and prev the cell
-    // before the first (< 0: none, the row starts here).  Returns false if it
-    // has more than 31 gaps.  Fills the root's tables and hands back the frame
+    // before the first (< 0: none, the row starts here).  The lanes in `lanes`
+    // call together.  Returns false if the root has more than 31 gaps.  Fills the root's tables and hands back the frame
     // in registers.
     //
     // One pass over the list in order, with no data-dependent branch so that
@@ -131,8 +130,8 @@ struct Tail {
     // different lengths.)  The face numbers of the gaps in U, one 16-bit word
     // per gap, are then turned into planes by a 16 x 16 bit transposition.
     template <class List, class WOf>
-    __device__ __forceinline__ bool setup(const List &L, int placed, int K0, const TailPages &pg,
-                                          WOf &&w, int prev, uint32_t &C, uint32_t (&W)[TMAX],
+    __device__ __forceinline__ bool setup(unsigned lanes, const List &L, int placed, int K0,
+                                          const TailPages &pg, WOf &&w, int prev, uint32_t &C, uint32_t (&W)[TMAX],
                                           uint32_t &R, uint32_t &H) const {
         uint16_t *pre = reinterpret_cast<uint16_t *>(area + Y::kPre) + lane;
         uint16_t *ids = reinterpret_cast<uint16_t *>(area + Y::kIds) + lane;
@@ -160,7 +159,7 @@ struct Tail {
             c = after;
         }
         // Not one cycle (cell 0 met again before the end): left to the list walk.
-        if (c != 0 || pos[0] != 0) return false;
+        const bool cycle = c == 0 && pos[0] == 0;
         // The faces of the w's on page b (a w has no arc there, so its gap is
         // in the face before it).
         uint32_t fw[TMAX];
@@ -178,6 +177,7 @@ struct Tail {
             }
         }
         const uint32_t fprev = prev >= 0 ? pre[prev * 32] : 0;
+        __syncwarp(lanes);  // the gap ids go over other lanes' `pre`
         // U in list order.
         uint64_t places = 0;
         int gaps = 0;
@@ -192,7 +192,7 @@ struct Tail {
             }
             gaps += in;
         }
-        if (gaps > 31) return false;
+        if (!cycle || gaps > 31) return false;
         uint32_t a[16];
 #pragma unroll
         for (int j = 0; j < 16; ++j) a[j] = word(Y::kGapIds)[j * 32 + lane];
