@@ -628,6 +628,26 @@ __device__ __forceinline__ int ring_claim(const Queue &Q, unsigned long long *co
     return __shfl_sync(kFull, got, 0);
 }
 
+// The run header read by one warp-wide load (lane k holds word k): every warp
+// polls the same line, and one request instead of one per field keeps its L2
+// slice from being the bottleneck of small jobs.
+struct HeaderView {
+    unsigned long long word;
+    __device__ __forceinline__ explicit HeaderView(const QueueHeader *hdr) {
+        const int lane = threadIdx.x & 31;
+        word = lane < 8 ? vload(reinterpret_cast<const unsigned long long *>(hdr) + lane) : 0;
+    }
+    __device__ __forceinline__ unsigned long long get(int k) const {
+        return __shfl_sync(kFull, word, k);
+    }
+    __device__ __forceinline__ unsigned long long init_next() const { return get(0); }
+    __device__ __forceinline__ unsigned long long spawn_head() const { return get(1); }
+    __device__ __forceinline__ unsigned long long spawn_tail() const { return get(2); }
+    __device__ __forceinline__ unsigned long long completed() const { return get(3); }
+    __device__ __forceinline__ unsigned int error() const { return static_cast<unsigned int>(get(5)); }
+    __device__ __forceinline__ long long idle_lanes() const { return static_cast<long long>(get(6)); }
+};
+
 // Called once per warp (lane 0) as it leaves a persistent launch, after all
 // of its counters are in.  Warps leave early on purpose (idle for wait_limit
 // rounds while others still work), so only the last warp out can tell

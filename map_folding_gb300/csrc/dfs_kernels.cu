@@ -116,9 +116,21 @@ __global__ void ring_init_kernel(unsigned long long *seq, unsigned long long cap
 }
 
 // Row counting (tail.cuh) of the persistent kernels.
-constexpr int kTailFill = 16;    // frames that make a level full
-constexpr int kTailRoots = 28;   // lanes at the row that start a count
-constexpr uint32_t kTailRounds = 8;  // bookkeeping rounds that a count stands for
+// Frames that make a level full, lanes at the row that start a count, and the
+// bookkeeping rounds that a count stands for (50,000 7x7 cases: 1,216 ms with
+// 16 / 24 / 16; fill 10: 1,312, fill 24: 1,257; roots 18: 1,294, roots 28:
+// 1,189; rounds 32: 1,232, rounds 8: 1,206).
+constexpr int kTailFill = 16;
+constexpr int kTailRoots = 28;
+constexpr uint32_t kTailRounds = 8;
+// Levels above the row from which a subtree may be handed out: below, an item
+// is a root or two and costs as much to pass on as to count (500 7x7 cases:
+// 32.1 ms at 2, 30.8 at 4, 30.0 at 6; 5x5 at depth 15: 2.46, 2.49, 3.68).
+constexpr int kRowSplit = 4;
+// Idle lanes of a working warp that go for split items between bookkeepings:
+// every attempt stops the warp for two trips to L2 (500 7x7 cases: 30.8 ms with
+// 1, 29.1 with 16; 6x6: 135 and 131 ms).
+constexpr int kTakeLanes = 16;
 constexpr int kNoRow = 1 << 20;
 constexpr int kRowLevels = 4;  // Lunnon: levels to go, of a map with rows, from which they pay
 
@@ -255,14 +267,19 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
     }
 
     // Prefetch state: 0 = no initial unit left for this lane, 1 = index
-    // taken.  The first indices come from one warp-aggregated atomicAdd.
+    // taken.  The first indices come from one warp-aggregated atomicAdd; with
+    // fewer units than lanes every warp takes its share of them, not the
+    // first warps 32 each.
+    const unsigned long long warps = (unsigned long long)gridDim.x * (TPB / 32);
+    const unsigned long long even = (num + warps - 1) / warps;
+    const int share = even < 32 ? int(even) : 32;
     unsigned long long pre_k = 0;
     {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&Q.hdr->init_next, 32ULL);
+        if (lane == 0) base = atomicAdd(&Q.hdr->init_next, (unsigned long long)share);
         pre_k = __shfl_sync(kFull, base, 0) + lane;
     }
-    int pre_stage = 1;
+    int pre_stage = lane < share ? 1 : 0;
     uint4 pre[kVecs];
     uint32_t pre_owner = 0;
 
@@ -338,21 +355,30 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         return got < want;
     };
 
-    // Warp-cooperative donation (all 32 lanes call): every busy lane with an
-    // untried sibling set at least kMinSplitHeight above the counted level
-    // gives the shallowest such set away.  One claim on the ring's tail
-    // reserves cells for all donors; each donor rolls its list back to that
-    // level, copies it out, replays, and publishes.
-    auto donate = [&]() {
+    // Warp-cooperative donation (all 32 lanes call): up to `quota` busy lanes
+    // with an untried sibling set high enough above the counted level give the
+    // shallowest such set away, those with the shallowest sets first.  One
+    // claim on the ring's tail reserves cells for all donors; each donor rolls
+    // its list back to that level, copies it out, replays, and publishes.
+    auto donate = [&](int quota) {
         int s = root;
         const uint64_t m = busy && !fresh ? shallowest_siblings(S, root, lvl, s) : 0;
-        const bool can = busy && !fresh && m != 0 && last - s >= kMinSplitHeight;
-        const unsigned donors = __ballot_sync(kFull, can);
+        const int low = TMAX > 0 && row_level != kNoRow ? row_level - s : last - s;
+        const bool can = busy && !fresh && m != 0 &&
+                         low >= (TMAX > 0 && row_level != kNoRow ? kRowSplit : kMinSplitHeight);
+        unsigned donors = 0;
+        for (int level = int(__reduce_min_sync(kFull, can ? unsigned(s) : 99u));
+             level < 99 && __popc(donors) < quota;) {
+            donors |= __ballot_sync(kFull, can && s == level);
+            level = int(__reduce_min_sync(kFull, can && s > level ? unsigned(s) : 99u));
+        }
+        while (__popc(donors) > quota) donors &= ~(1u << (31 - __clz(int(donors))));
         if (!donors) return;
+        const bool give = (donors >> lane) & 1u;
         unsigned long long first = 0;
         const int got = ring_claim(Q, &Q.hdr->spawn_tail, __popc(donors), false, first);
         const int rank = __popc(donors & lt_mask);
-        if (!can || rank >= got) return;
+        if (!give || rank >= got) return;
         roll_back(L, S, s, lvl);
         uint32_t w[24];
 #pragma unroll
@@ -424,7 +450,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         // says the ring has some (refreshed at bookkeeping, cleared by a miss).
         if (ring_hint) {
             const unsigned need = __ballot_sync(kFull, !busy && pre_stage == 0);
-            if (need && take_splits(need)) ring_hint = false;
+            if (need && (__popc(need) >= kTakeLanes || round + 1 >= period) && take_splits(need))
+                ring_hint = false;
         }
         const bool bookkeeping = ++round >= period;
         if (!__any_sync(kFull, busy)) {
@@ -440,7 +467,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                 }
             }
             const unsigned need = __ballot_sync(kFull, pre_stage == 0);
-            if (need) take_splits(need);
+            const HeaderView now(Q.hdr);
+            if (need && now.spawn_tail() != now.spawn_head()) take_splits(need);
             // A lane still holding a prefetched unit keeps the warp alive.
             const bool holding = __any_sync(kFull, pre_stage != 0 && pre_k < num);
             if (__any_sync(kFull, busy) || holding) {
@@ -448,14 +476,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                 nap = 256;
                 continue;
             }
-            int stop = 0;
-            if (lane == 0) {
-                const unsigned long long total = num + vload(&Q.hdr->spawn_tail);
-                stop = (vload(&Q.hdr->init_next) >= num && vload(&Q.hdr->completed) >= total) ||
-                       *reinterpret_cast<volatile unsigned int *>(&Q.hdr->error) != 0u ||
-                       ++idle_rounds > wait_limit;
-            }
-            stop = __shfl_sync(kFull, stop, 0);
+            const bool stop = (now.init_next() >= num && now.completed() >= num + now.spawn_tail()) ||
+                              now.error() != 0u || ++idle_rounds > wait_limit;
             if (stop) break;
             __nanosleep(nap);
             if (nap < 8192) nap <<= 1;
@@ -540,7 +562,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         const unsigned idle_mask = __ballot_sync(kFull, !busy);
         const unsigned long long f = warp_sum(finished);
         finished = 0;
-        long long want = 0, queued = 0;
+        long long queued = 0;
+        int quota = 0;
         if (lane == 0) {
             if (f) atomicAdd(&Q.hdr->completed, f);
             const int idle_now = __popc(idle_mask);
@@ -549,17 +572,25 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                           (unsigned long long)(long long)(idle_now - reported_idle));
                 reported_idle = idle_now;
             }
-            if (vload(&Q.hdr->init_next) >= num) {
-                queued = (long long)(vload(&Q.hdr->spawn_tail) - vload(&Q.hdr->spawn_head));
-                const long long waiting = *reinterpret_cast<volatile long long *>(&Q.hdr->idle_lanes);
-                want = waiting - queued;
+        }
+        const HeaderView now(Q.hdr);
+        if (now.init_next() >= num) {
+            queued = (long long)(now.spawn_tail() - now.spawn_head());
+            const long long waiting = now.idle_lanes();
+            const long long want = waiting - queued;
+            if (want > 0) {
+                // This warp's share of what is wanted, twice over: every warp
+                // with work sees the same number, and if all gave all they
+                // could the ring would fill with crumbs.
+                const long long givers = (long long)warps - waiting / 32;
+                const long long q = givers > 0 ? (2 * want + givers - 1) / givers : 32;
+                quota = q < 32 ? int(q) : 32;
             }
         }
-        want = __shfl_sync(kFull, want, 0);
-        ring_hint = __shfl_sync(kFull, queued, 0) > 0;
+        ring_hint = queued > 0;
         // Feed waiting lanes: busy lanes give away their shallowest untried
         // siblings while lanes wait for work.
-        if (want > 0) donate();
+        if (quota > 0) donate(quota);
     }
 #undef MF_FETCH_RECORD
 

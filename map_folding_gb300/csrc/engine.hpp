@@ -171,7 +171,7 @@ struct QueueHeader {
     long long idle_lanes;           // lanes waiting for work (warps report deltas)
     unsigned long long warps_out;   // warps that have left the launch
 };
-static_assert(sizeof(QueueHeader) == 64, "queue header layout");
+static_assert(sizeof(QueueHeader) == 64, "queue header layout");  // read as 8 words by HeaderView
 
 // Error words of a persistent launch (QueueHeader::error).
 constexpr unsigned int kErrMalformed = 1;  // a unit's list was not a permutation
