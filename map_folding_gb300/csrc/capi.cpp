@@ -1306,7 +1306,13 @@ uint32_t mf_solve_cases(uint32_t n, uint32_t start_i, uint32_t stop_i, const uin
     std::vector<uint64_t> counts(case_count + 1);
     mf_run_stats st{};
     if (case_count) {
-        int rc = count_cases_host(int(n), int(start_i), int(stop_i), cycles.data(), case_count, 0,
+        // The plain kernel is one launch and shares a case among 32 lanes; from
+        // 13 levels on a heavy case is worth more than a warp and the batched
+        // kernel splits it (64 / 256 7x7 cases of 14 cells, plain and batched:
+        // to 24 cells 292 / 458 and 485 / 769 us, to 26 519 / 899 and 607 /
+        // 805 us, to 28 1.70 / 4.12 and 1.09 / 1.72 ms).
+        const int mode = stop_i - start_i >= 13 ? 1 : 0;
+        int rc = count_cases_host(int(n), int(start_i), int(stop_i), cycles.data(), case_count, mode,
                                   nullptr, counts.data(), &st, nullptr);
         if (rc) return write(0, 0, 3);
     }

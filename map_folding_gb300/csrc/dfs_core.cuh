@@ -406,22 +406,116 @@ __device__ __forceinline__ void init_stack(LocalStack &S, uint8_t *, size_t) {
     S.base = 0;
 }
 
-// Run one loaded unit per lane to completion in lockstep rounds (no refill):
-// the plain one-thread-per-unit kernels.  Walks are resumable and take at
-// most kWalkCap steps per round.
+// The n-th set bit of m (n < popcount of m).
+__device__ __forceinline__ int nth_bit(unsigned m, int n) {
+    int at = 0;
+#pragma unroll
+    for (int w = 16; w >= 1; w >>= 1) {
+        const int below = __popc((m >> at) & ((1u << w) - 1));
+        if (n >= below) {
+            n -= below;
+            at += w;
+        }
+    }
+    return at;
+}
+
+// Of the lanes with `can`, up to `quota` with the smallest `s` (all 32 lanes
+// call).
+__device__ __forceinline__ unsigned shallowest_lanes(bool can, int s, int quota) {
+    unsigned lanes = 0;
+    for (int level = int(__reduce_min_sync(kFull, can ? unsigned(s) : 99u));
+         level < 99 && __popc(lanes) < quota;) {
+        lanes |= __ballot_sync(kFull, can && s == level);
+        level = int(__reduce_min_sync(kFull, can && s > level ? unsigned(s) : 99u));
+    }
+    while (__popc(lanes) > quota) lanes &= ~(1u << (31 - __clz(int(lanes))));
+    return lanes;
+}
+
+// Sharing within the warp (all 32 lanes call): busy lanes hand their
+// shallowest untried siblings straight to the `idle` lanes, list by list in
+// shared memory, without a trip to L2.  A lane may give what it has at levels
+// up to `floor`.  around(from, take) runs on all lanes in between: `from` is
+// the giver of a lane with `take`, and whatever else goes over is shuffled
+// there; begin(level, mask) then runs on the taking lanes.  Returns false if
+// no lane has anything to give.
+template <class List, class Stk, class Around, class Begin>
+__device__ __forceinline__ bool share_in_warp(const List &L, Stk &S, bool searching, int root,
+                                              int lvl, int floor, unsigned idle, Around &&around,
+                                              Begin &&begin) {
+    const int lane = threadIdx.x & 31;
+    int s = root;
+    const uint64_t m = searching ? shallowest_siblings(S, root, lvl, s) : 0;
+    const unsigned donors = shallowest_lanes(m != 0 && s <= floor, s, __popc(idle));
+    const int n = __popc(donors);
+    if (n == 0) return false;
+    const bool give = (donors >> lane) & 1u;
+    const int rank = __popc(idle & ((1u << lane) - 1u));
+    const bool take = ((idle >> lane) & 1u) && rank < n;
+    const int from = take ? nth_bit(donors, rank) : lane;
+    if (give) roll_back(L, S, s, lvl);
+    __syncwarp();
+    const int level = __shfl_sync(kFull, s, from);
+    const uint64_t mask = __shfl_sync(kFull, m, from);
+    around(from, take);
+    if (take) {
+        const List theirs{L.base + 4 * (from - lane)};
+        for (int j = 0; j < level; ++j) L.put(j, theirs.get(j));
+        begin(level, mask);
+    }
+    __syncwarp();
+    if (give) replay_keeping_pick(L, S, s, lvl);
+    return true;
+}
+
+// Lanes without work that make a warp share (100 us of a 19 ms job at 4), and
+// how high above the counted level a piece must start.
+constexpr int kShareLanes = 2;
+constexpr int kMinShareHeight = 2;
+
+// Run the loaded units of a warp to completion in lockstep rounds (no refill):
+// the plain kernels.  A lane whose unit is done takes pieces of the others',
+// so the heaviest unit of a warp no longer sets its time; `acc` holds 32
+// counters of the warp in shared memory for what others counted of a lane's
+// unit.  Walks are resumable and take at most kWalkCap steps per round.
+// Returns the leaves of the lane's own unit.
 template <class Rules, class Stk, int TPB>
-__device__ __forceinline__ void run_units(const Rules &R, const List<TPB> &L, Stk &S, bool busy,
-                                          int root, int last, unsigned long long &leaves,
-                                          unsigned long long &nodes) {
-    int lvl = root, eval = root;
+__device__ __forceinline__ unsigned long long run_units(const Rules &R, const List<TPB> &L, Stk &S,
+                                                        bool busy, int root, int last,
+                                                        unsigned long long *acc,
+                                                        unsigned long long &nodes) {
+    const int lane = threadIdx.x & 31;
+    int lvl = root, eval = root, owner = lane;
     bool fresh = true;
+    unsigned long long own = 0, leaves = 0;
+    acc[lane] = 0;
+    __syncwarp();
     if (busy && root > last) {  // nothing left to place: one completion
-        leaves += 1;
+        own = 1;
         busy = false;
     }
-    bool walking = false;
+    bool walking = false, miss = false;
     typename Rules::Walk w;
-    while (__any_sync(kFull, busy)) {
+    for (int round = 0;; ++round) {
+        const unsigned idle = __ballot_sync(kFull, !busy);
+        if (idle == kFull) break;
+        if (!(round & 15)) miss = false;
+        if (__popc(idle) >= kShareLanes && !miss) {
+            int whose = 0;
+            miss = !share_in_warp(
+                L, S, busy && !fresh, root, lvl, last - kMinShareHeight, idle,
+                [&](int from, bool) { whose = __shfl_sync(kFull, owner, from); },
+                [&](int level, uint64_t mask) {
+                    owner = whose;
+                    root = level;
+                    S.set(root, mask);
+                    eval = advance(L, S, lvl, root);
+                    walking = false;
+                    fresh = false;
+                    busy = true;
+                });
+        }
         if (busy) {
             if (!walking) {
                 R.begin(L, eval, nodes, w);
@@ -433,9 +527,16 @@ __device__ __forceinline__ void run_units(const Rules &R, const List<TPB> &L, St
                 eval = apply_advance(L, S, lvl, eval, root, last, fresh, g, leaves);
                 fresh = false;
                 busy = eval >= 0;
+                if (!busy) {
+                    if (owner == lane) own += leaves;
+                    else if (leaves) atomicAdd(acc + owner, leaves);
+                    leaves = 0;
+                }
             }
         }
     }
+    __syncwarp();
+    return own + acc[lane];
 }
 
 // ---------------------------------------------------------- sym tables ---

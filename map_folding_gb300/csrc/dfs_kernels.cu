@@ -40,12 +40,17 @@ namespace {
 
 // ------------------------------------------------------- plain kernels ---
 
-// One thread per case: d_counts[k] = completions of case k (UINT64_MAX if
-// its cycle is malformed).  Shared memory: 4 edge pages, then the carve.
+// The plain kernels: each warp takes `per_warp` consecutive units, one a lane
+// (32, or fewer where there are too few units to give every resident warp 32),
+// and its lanes share what is left when theirs are done (run_units).  8,191
+// states of the 5x5 map at depth 15, one lane each to the end, took 7.9 ms.
+
+// d_counts[k] = completions of case k (UINT64_MAX if its cycle is malformed).
+// Shared memory: sym tables and hop rows, the carve, the warps' counters.
 template <int TPB, int LEVELS>
 __global__ void __launch_bounds__(TPB)
     sym_plain_kernel(const uint8_t *__restrict__ edges, int start_i, int stop_i,
-                     const uint8_t *__restrict__ cycles, uint64_t num,
+                     const uint8_t *__restrict__ cycles, uint64_t num, int per_warp,
                      unsigned long long *__restrict__ counts,
                      unsigned long long *__restrict__ nodes_out) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -55,14 +60,18 @@ __global__ void __launch_bounds__(TPB)
     const List<TPB> L = C::list(smem, tables);
     typename StackOf<TPB, LEVELS>::type S;
     init_stack<TPB, 16, LEVELS>(S, smem, tables);
-    const uint64_t unit = uint64_t(blockIdx.x) * TPB + threadIdx.x;
-    const bool active = unit < num;
+    const int lane = threadIdx.x & 31;
+    const uint64_t unit = (uint64_t(blockIdx.x) * (TPB / 32) + threadIdx.x / 32) * per_warp + lane;
+    const bool active = lane < per_warp && unit < num;
     if (active) load_list<TPB, 16>(L, cycles + unit * kSymCells, kSymCells);
 
-    unsigned long long nodes = 0, leaves = 0;
+    unsigned long long nodes = 0;
     const bool bad = active && !list_valid(L, start_i);
     S.base = start_i;
-    run_units(R, L, S, active && !bad, start_i, stop_i - 1, leaves, nodes);
+    auto *acc = reinterpret_cast<unsigned long long *>(smem + tables + C::kThreadBytes) +
+                (threadIdx.x & ~31);
+    const unsigned long long leaves =
+        run_units(R, L, S, active && !bad, start_i, stop_i - 1, acc, nodes);
     if (active) counts[unit] = bad ? ~0ULL : leaves;
     if (nodes_out) {
         const unsigned long long s = warp_sum(nodes);
@@ -70,13 +79,12 @@ __global__ void __launch_bounds__(TPB)
     }
 }
 
-// One thread per prefix state.  Shared memory: the map's neighbour table,
-// then the carve.
+// Shared memory: the map's neighbour table, the carve, the warps' counters.
 template <int TPB, int LEVELS>
 __global__ void __launch_bounds__(TPB)
     lunnon_plain_kernel(const uint8_t *__restrict__ table, int table_bytes, int n, int dim,
                         int start_leaf, const uint8_t *__restrict__ states, uint32_t stride,
-                        uint64_t num, unsigned long long *__restrict__ per_state,
+                        uint64_t num, int per_warp, unsigned long long *__restrict__ per_state,
                         unsigned long long *__restrict__ total,
                         unsigned long long *__restrict__ nodes_out) {
     extern __shared__ __align__(16) uint8_t smem[];
@@ -86,15 +94,19 @@ __global__ void __launch_bounds__(TPB)
     const List<TPB> L = C::list(smem, table_bytes);
     typename StackOf<TPB, LEVELS>::type S;
     init_stack<TPB, 17, LEVELS>(S, smem, table_bytes);
-    const uint64_t unit = uint64_t(blockIdx.x) * TPB + threadIdx.x;
-    const bool active = unit < num;
+    const int lane = threadIdx.x & 31;
+    const uint64_t unit = (uint64_t(blockIdx.x) * (TPB / 32) + threadIdx.x / 32) * per_warp + lane;
+    const bool active = lane < per_warp && unit < num;
     if (active) load_list<TPB, 17>(L, states + unit * stride, stride);
     __syncthreads();
 
-    unsigned long long nodes = 0, leaves = 0;
+    unsigned long long nodes = 0;
     const bool bad = active && !list_valid(L, start_leaf < n + 1 ? start_leaf : n + 1);
     S.base = start_leaf;
-    run_units(LunnonRules{smem, n, dim}, L, S, active && !bad, start_leaf, n, leaves, nodes);
+    auto *acc = reinterpret_cast<unsigned long long *>(smem + table_bytes + C::kThreadBytes) +
+                (threadIdx.x & ~31);
+    unsigned long long leaves = run_units(LunnonRules{smem, n, dim}, L, S, active && !bad,
+                                          start_leaf, n, acc, nodes);
     leaves = bad ? 0 : leaves * static_cast<unsigned long long>(n);
     if (active && per_state) per_state[unit] = bad ? ~0ULL : leaves;
     if (total) {
@@ -124,9 +136,12 @@ constexpr int kTailFill = 16;
 constexpr int kTailRoots = 28;
 constexpr uint32_t kTailRounds = 8;
 // Levels above the row from which a subtree may be handed out: below, an item
-// is a root or two and costs as much to pass on as to count (500 7x7 cases:
-// 32.1 ms at 2, 30.8 at 4, 30.0 at 6; 5x5 at depth 15: 2.46, 2.49, 3.68).
-constexpr int kRowSplit = 4;
+// is a root or two and costs as much to pass on as to count (4x5 at
+// depth 12, with sharing within the warp: 310 us at 4, 244 at 6).
+constexpr int kRowSplit = 5;
+// ... and above the counted level where no row is counted by itself.
+constexpr int kMinRingHeight = 6;
+constexpr int kRowShare = 1;  // the same for a piece shared within the warp
 // Idle lanes of a working warp that go for split items between bookkeepings:
 // every attempt stops the warp for two trips to L2 (500 7x7 cases: 30.8 ms with
 // 1, 29.1 with 16; 6x6: 135 and 131 ms).
@@ -239,6 +254,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     bool busy = false, fresh = false;
+    bool whole = true;     // a unit or split item, not a piece shared within the warp
     bool walking = false;  // a resumable walk is under way
     SymHopRules::Walk swalk{};
     LunnonRules::Walk lwalk{};
@@ -272,14 +288,14 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
     // first warps 32 each.
     const unsigned long long warps = (unsigned long long)gridDim.x * (TPB / 32);
     const unsigned long long even = (num + warps - 1) / warps;
-    const int share = even < 32 ? int(even) : 32;
+    const int own = even < 32 ? int(even) : 32;
     unsigned long long pre_k = 0;
     {
         unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(&Q.hdr->init_next, (unsigned long long)share);
+        if (lane == 0) base = atomicAdd(&Q.hdr->init_next, (unsigned long long)own);
         pre_k = __shfl_sync(kFull, base, 0) + lane;
     }
-    int pre_stage = lane < share ? 1 : 0;
+    int pre_stage = lane < own ? 1 : 0;
     uint4 pre[kVecs];
     uint32_t pre_owner = 0;
 
@@ -298,7 +314,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             atomicAdd(counts + owner, leaves * weight);
         }
         leaves = 0;
-        ++finished;
+        if (whole) ++finished;
     };
 
     int row_len = 0;  // Lunnon: leaves of a row of the map
@@ -338,6 +354,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             for (int k2 = 0; k2 < WORDS; ++k2) L.set_word(k2, w[k2]);
             owner = w[17];
             root = int(w[20]);
+            whole = true;
             if (kSym) {
                 last = sym.last;
                 S.base = sym.start_i;
@@ -365,14 +382,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         const uint64_t m = busy && !fresh ? shallowest_siblings(S, root, lvl, s) : 0;
         const int low = TMAX > 0 && row_level != kNoRow ? row_level - s : last - s;
         const bool can = busy && !fresh && m != 0 &&
-                         low >= (TMAX > 0 && row_level != kNoRow ? kRowSplit : kMinSplitHeight);
-        unsigned donors = 0;
-        for (int level = int(__reduce_min_sync(kFull, can ? unsigned(s) : 99u));
-             level < 99 && __popc(donors) < quota;) {
-            donors |= __ballot_sync(kFull, can && s == level);
-            level = int(__reduce_min_sync(kFull, can && s > level ? unsigned(s) : 99u));
-        }
-        while (__popc(donors) > quota) donors &= ~(1u << (31 - __clz(int(donors))));
+                         low >= (TMAX > 0 && row_level != kNoRow ? kRowSplit : kMinRingHeight);
+        const unsigned donors = shallowest_lanes(can, s, quota);
         if (!donors) return;
         const bool give = (donors >> lane) & 1u;
         unsigned long long first = 0;
@@ -394,6 +405,39 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         ring_put(Q, first + rank, w);
     };
 
+    // Pieces shared within the warp are no work items of their own: a piece
+    // belongs to its unit's count and to nobody's bookkeeping.
+    auto share = [&](unsigned idle) -> bool {
+        uint32_t whose = 0;
+        int its_row = 0;
+        return share_in_warp(
+            L, S, busy && !fresh, root, lvl,
+            TMAX > 0 && row_level != kNoRow ? row_level - kRowShare : last - kMinShareHeight, idle,
+            [&](int from, bool) {
+                whose = __shfl_sync(kFull, owner, from);
+                its_row = __shfl_sync(kFull, row_level, from);
+            },
+            [&](int level, uint64_t mask) {
+                owner = whose;
+                root = level;
+                if (kSym) {
+                    last = sym.last;
+                    S.base = sym.start_i;
+                    row_level = its_row;
+                } else {
+                    set_instance(owner);
+                }
+                S.set(root, mask);
+                eval = advance(L, S, lvl, root);
+                whole = false;
+                walking = false;
+                by_walk = false;
+                fresh = false;
+                busy = true;
+            });
+    };
+
+    bool share_miss = false;  // warp-uniform: nothing to share at the last try
     uint32_t nap = 256;  // idle back-off, ns
     for (;;) {
         // Start the prefetched unit on lanes whose search has ended.
@@ -408,6 +452,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                         if (4 * q + k < WORDS) L.set_word(4 * q + k, ws[k]);
                 }
                 ++started;
+                whole = true;
                 bool ok;
                 if (kSym) {
                     owner = uint32_t(pre_k);
@@ -446,6 +491,9 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                 pre_stage = 0;
             }
         }
+        // Idle lanes share the busy lanes' work.
+        const unsigned unfed = __ballot_sync(kFull, !busy && pre_stage == 0);
+        if (__popc(unfed) >= kShareLanes && unfed != kFull && !share_miss) share_miss = !share(unfed);
         // Lanes without initial units take split items while the warp's hint
         // says the ring has some (refreshed at bookkeeping, cleared by a miss).
         if (ring_hint) {
@@ -588,6 +636,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             }
         }
         ring_hint = queued > 0;
+        share_miss = false;
         // Feed waiting lanes: busy lanes give away their shallowest untried
         // siblings while lanes wait for work.
         if (quota > 0) donate(quota);
@@ -789,12 +838,19 @@ cudaError_t reset_queue(const Queue &Q, cudaStream_t stream) {
 
 }  // namespace
 
+// Units per warp of a plain launch of CTAs of `tpb` threads, `bpsm` of them
+// resident on an SM.
+static int plain_units_per_warp(uint64_t num, int bpsm, int tpb) {
+    const uint64_t warps = uint64_t(device_sm_count()) * uint64_t(bpsm) * uint64_t(tpb / 32);
+    const uint64_t k = (num + warps - 1) / (warps ? warps : 1);
+    return k < 1 ? 1 : (k > 32 ? 32 : int(k));
+}
+
 cudaError_t launch_sym_plain(const uint8_t *d_edges, int start_i, int stop_i,
                              const uint8_t *d_cycles, uint64_t num, uint64_t *d_counts,
                              uint64_t *d_nodes, cudaStream_t stream) {
     if (num == 0) return cudaSuccess;
     constexpr int TPB = 128;
-    const uint64_t blocks = (num + TPB - 1) / TPB;
     const int levels = pick_levels(stop_i - 1 - start_i);
     const size_t tables = sym_tables_bytes(stop_i - start_i);
     auto *counts = reinterpret_cast<unsigned long long *>(d_counts);
@@ -802,11 +858,13 @@ cudaError_t launch_sym_plain(const uint8_t *d_edges, int start_i, int stop_i,
     int bpsm = 0;
 #define MF_SYM_PLAIN(LV)                                                                        \
     do {                                                                                        \
-        const size_t smem = tables + Carve<TPB, 16, LV>::kThreadBytes;                          \
+        const size_t smem = tables + Carve<TPB, 16, LV>::kThreadBytes + 8 * TPB;                \
         cudaError_t e = prepare(sym_plain_kernel<TPB, LV>, smem, TPB, 0, bpsm);                 \
         if (e != cudaSuccess) return e;                                                         \
+        const int per = plain_units_per_warp(num, bpsm, TPB);                                   \
+        const uint64_t blocks = (num + per * (TPB / 32) - 1) / (per * (TPB / 32));              \
         sym_plain_kernel<TPB, LV><<<unsigned(blocks), TPB, smem, stream>>>(                     \
-            d_edges, start_i, stop_i, d_cycles, num, counts, nodes);                            \
+            d_edges, start_i, stop_i, d_cycles, num, per, counts, nodes);                       \
     } while (0)
     switch (levels) {
         case 24: MF_SYM_PLAIN(24); break;
@@ -826,18 +884,20 @@ cudaError_t launch_lunnon_plain(const uint8_t *d_table, int n, int dim, int star
     constexpr int TPB = 128;
     const int table_bytes = (dim * (n + 1) * (n + 1) + 15) / 16 * 16;
     const int levels = pick_levels(n - start_leaf);
-    const uint64_t blocks = (num + TPB - 1) / TPB;
     auto *per = reinterpret_cast<unsigned long long *>(d_per_state);
     auto *tot = reinterpret_cast<unsigned long long *>(d_total);
     auto *nodes = reinterpret_cast<unsigned long long *>(d_nodes);
     int bpsm = 0;
 #define MF_LUN_PLAIN(LV)                                                                        \
     do {                                                                                        \
-        const size_t smem = table_bytes + Carve<TPB, 17, LV>::kThreadBytes;                     \
+        const size_t smem = table_bytes + Carve<TPB, 17, LV>::kThreadBytes + 8 * TPB;           \
         cudaError_t e = prepare(lunnon_plain_kernel<TPB, LV>, smem, TPB, 0, bpsm);              \
         if (e != cudaSuccess) return e;                                                         \
+        const int k = plain_units_per_warp(num, bpsm, TPB);                                     \
+        const uint64_t blocks = (num + k * (TPB / 32) - 1) / (k * (TPB / 32));                  \
         lunnon_plain_kernel<TPB, LV><<<unsigned(blocks), TPB, smem, stream>>>(                  \
-            d_table, table_bytes, n, dim, start_leaf, d_states, stride, num, per, tot, nodes);   \
+            d_table, table_bytes, n, dim, start_leaf, d_states, stride, num, k, per, tot,       \
+            nodes);                                                                             \
     } while (0)
     switch (levels) {
         case 24: MF_LUN_PLAIN(24); break;
