@@ -335,12 +335,13 @@ int32_t mf_lunnon_count_range(const mf_lunnon_plan *cplan, int32_t depth, uint64
     if (rc) return rc;
     const double t0 = now_seconds();
     const uint32_t stride = lunnon_state_stride(plan->t.n);
-    const uint64_t all = collect_lunnon_states(plan->t, depth, nullptr, 0, stride);
+    const LunnonStates states(plan->t, depth);
+    const uint64_t all = states.total();
     uint64_t total = all > first_state ? all - first_state : 0;
     if (max_states && max_states < total) total = max_states;
     auto *h_states = static_cast<uint8_t *>(scratch(kHostUnits, total * stride, true));
     if (!h_states) return MF_ERR_CUDA;
-    collect_lunnon_states(plan->t, depth, h_states, total, stride, first_state);
+    states.write(first_state, total, h_states, stride);
     const double t1 = now_seconds();
     auto *d_states = static_cast<uint8_t *>(scratch(kDevUnits, total * stride, false));
     auto *d_acc = static_cast<uint64_t *>(scratch(kDevCounts, 2 * sizeof(uint64_t), false));
@@ -395,6 +396,8 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
     std::vector<LunnonInstanceDev> inst(num_plans);
     std::vector<uint8_t> tables;
     std::vector<uint64_t> per_plan(num_plans), first(num_plans, 0);
+    std::vector<LunnonStates> states;
+    states.reserve(num_plans);
     uint64_t total = 0;
     for (int k = 0; k < num_plans; ++k) {
         const mf_lunnon_plan *p = plans[k];
@@ -412,7 +415,8 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
         inst[k].row = last_row(p->t);
         tables.insert(tables.end(), p->t.next.begin(), p->t.next.end());
         tables.resize((tables.size() + 15) / 16 * 16, 0);
-        const uint64_t all = collect_lunnon_states(p->t, d, nullptr, 0, stride);
+        states.emplace_back(p->t, d);
+        const uint64_t all = states.back().total();
         first[k] = firsts ? firsts[k] : 0;
         per_plan[k] = all > first[k] ? all - first[k] : 0;
         if (limits && limits[k] && limits[k] < per_plan[k]) per_plan[k] = limits[k];
@@ -430,8 +434,7 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
     auto *h_owner = reinterpret_cast<uint32_t *>(h_units + unit_bytes);
     uint64_t at = 0;
     for (int k = 0; k < num_plans; ++k) {
-        collect_lunnon_states(plans[k]->t, inst[k].start_leaf - 1, h_units + at * stride,
-                              per_plan[k], stride, first[k]);
+        states[k].write(first[k], per_plan[k], h_units + at * stride, stride);
         for (uint64_t s = 0; s < per_plan[k]; ++s) h_owner[at + s] = uint32_t(k);
         at += per_plan[k];
     }
@@ -652,6 +655,8 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
     std::vector<LunnonInstanceDev> inst(num_plans);
     std::vector<uint8_t> meta;
     std::vector<uint64_t> per_plan(num_plans);
+    std::vector<LunnonStates> states;
+    states.reserve(num_plans);
     uint64_t total = 0;
     int max_levels = 0, row_levels = 0;
     for (int k = 0; k < num_plans; ++k) {
@@ -666,7 +671,8 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
         inst[k] = LunnonInstanceDev{uint32_t(meta.size()), p->t.n, p->t.dim, d + 1, last_row(p->t)};
         meta.insert(meta.end(), p->t.next.begin(), p->t.next.end());
         meta.resize((meta.size() + 15) / 16 * 16, 0);
-        per_plan[k] = collect_lunnon_states(p->t, d, nullptr, 0, stride);
+        states.emplace_back(p->t, d);
+        per_plan[k] = states.back().total();
         total += per_plan[k];
         max_levels = std::max(max_levels, p->t.n - d - 1);
         if (inst[k].row) row_levels = std::max(row_levels, p->t.n - d - 1);
@@ -683,8 +689,7 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
     auto *owner = reinterpret_cast<uint32_t *>(host.data() + unit_bytes);
     uint64_t at = 0;
     for (int k = 0; k < num_plans; ++k) {
-        collect_lunnon_states(plans[k]->t, inst[k].start_leaf - 1, host.data() + at * stride,
-                              per_plan[k], stride);
+        states[k].write(0, per_plan[k], host.data() + at * stride, stride);
         for (uint64_t s = 0; s < per_plan[k]; ++s) owner[at + s] = uint32_t(k);
         at += per_plan[k];
     }

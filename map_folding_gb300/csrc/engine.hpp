@@ -46,6 +46,25 @@ bool build_lunnon_tables(const int32_t *dims, int ndim, LunnonTables &t, std::st
 // Bytes per packed prefix-state record (b[0..n], padded to 16).
 inline uint32_t lunnon_state_stride(int n) { return uint32_t((n + 1 + 15) / 16 * 16); }
 
+// The prefix states at leaf depth `depth`, counted when made; write() writes
+// the records with index in [first, first + count), `stride` bytes each, in
+// the reference's emission order.
+class LunnonStates {
+  public:
+    LunnonStates(const LunnonTables &t, int depth);
+    uint64_t total() const { return first_.back(); }
+    void write(uint64_t first, uint64_t count, uint8_t *out, uint32_t stride) const;
+
+  private:
+    template <class F>
+    void each(size_t lo, size_t hi, F &&run) const;
+    const LunnonTables &t_;
+    int depth_ = 0, split_ = 0;
+    std::vector<uint8_t> roots_;   // states at depth split_, n + 1 bytes each
+    std::vector<uint64_t> first_;  // index of each root's first state; the total
+    std::vector<uint8_t> kept_;    // all states, where they are few
+};
+
 // Prefix states at leaf depth `depth` in the reference's emission order.
 // Writes the records with index in [first, first + cap), `stride` bytes
 // each; returns the total number of states.

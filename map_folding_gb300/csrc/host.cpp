@@ -4,11 +4,13 @@
 // runs on the host; the counting itself runs in the kernels (dfs_kernels.cu).
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <chrono>
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
 #include <set>
+#include <system_error>
 #include <thread>
 #include <unordered_set>
 
@@ -101,90 +103,172 @@ int default_lunnon_depth(const LunnonTables &t) {
 
 namespace {
 
+size_t host_threads() {
+    const unsigned hw = std::thread::hardware_concurrency();
+    return hw ? hw : 1;
+}
+
 // One level of the host search: the surviving gap positions for the leaf of
 // this level, in the order mf.c:118-124 leaves them on its stack; the search
 // consumes them from the end (mf.c:137, `gap[--g]`).
 struct GapFrame {
     uint8_t pos[MF_MAX_LEAVES + 1];
-    int count = 0;
     int left = 0;
 };
 
-void compute_frame(const LunnonTables &t, const uint8_t *b, int l, GapFrame &f, int *hits) {
-    f.count = 0;
-    uint8_t order[MF_MAX_LEAVES + 1];
-    int distinct = 0;
-    int bound = 0;
+// The gaps common to all constrained dimensions come in the order in which
+// the first of them walks its own, so the others are only masks.  Position 0
+// is dropped from l = 2 on: the normal-form filter (mf.c:83) prunes it.
+void compute_frame(const LunnonTables &t, const uint8_t *b, int l, GapFrame &f) {
+    f.left = 0;
+    int lead = -1;
+    uint64_t common = l >= 2 ? ~1ULL : ~0ULL;
     for (int i = 0; i < t.dim; ++i) {
-        int m = t.at(i, l, l);
-        if (m == l) continue;
-        ++bound;
-        while (m != l) {
-            if (hits[m]++ == 0) order[distinct++] = uint8_t(m);
-            m = t.at(i, l, b[m]);
+        const uint8_t *next = &t.next[(size_t(i) * (t.n + 1) + l) * (t.n + 1)];
+        if (next[l] == l) continue;
+        if (lead < 0) {
+            lead = i;
+            continue;
         }
+        uint64_t walked = 0;
+        for (int m = next[l]; m != l; m = next[b[m]]) walked |= 1ULL << m;
+        common &= walked;
     }
-    if (bound == 0) {
-        for (int m = 0; m < l; ++m) f.pos[f.count++] = uint8_t(m);
-    } else {
-        for (int k = 0; k < distinct; ++k) {
-            int m = order[k];
-            if (hits[m] == bound) f.pos[f.count++] = uint8_t(m);
-            hits[m] = 0;
-        }
+    if (lead < 0) {
+        for (int m = 0; m < l; ++m)
+            if ((common >> m) & 1) f.pos[f.left++] = uint8_t(m);
+        return;
     }
-    f.left = f.count;
+    const uint8_t *next = &t.next[(size_t(lead) * (t.n + 1) + l) * (t.n + 1)];
+    for (int m = next[l]; m != l; m = next[b[m]])
+        if ((common >> m) & 1) f.pos[f.left++] = uint8_t(m);
 }
 
-}  // namespace
-
-uint64_t collect_lunnon_states(const LunnonTables &t, int depth, uint8_t *out, uint64_t cap,
-                               uint32_t stride, uint64_t first) {
-    const int n = t.n;
-    if (depth < 0) depth = 0;
-    if (depth > n) depth = n;
-    uint8_t a[MF_MAX_LEAVES + 2] = {0};
-    uint8_t b[MF_MAX_LEAVES + 2] = {0};
-    int hits[MF_MAX_LEAVES + 2] = {0};
-    std::vector<GapFrame> frames(n + 2);
-    uint64_t found = 0;
-
-    auto enter = [&](int l) {
-        GapFrame &f = frames[l];
-        f.count = f.left = 0;
-        if (l >= 2 && b[0] != 1) return;  // normal-form filter, mf.c:83
-        if (l > depth) {
-            if (out != nullptr && found >= first && found - first < cap) {
-                uint8_t *rec = out + (found - first) * stride;
-                std::memset(rec, 0, stride);
-                std::memcpy(rec, b, size_t(n) + 1);
-            }
-            ++found;
-            return;
-        }
-        compute_frame(t, b, l, f, hits);
-    };
-
-    int l = 1;
-    enter(1);
+// Every descendant of the state b (leaves 1..from placed) at `depth` leaves,
+// in emission order; emit(b) returns false to stop.
+template <class F>
+void expand_states(const LunnonTables &t, uint8_t *b, int from, int depth, F &&emit) {
+    if (from >= depth) {
+        emit(b);
+        return;
+    }
+    GapFrame frames[MF_MAX_LEAVES + 2];
+    uint8_t after[MF_MAX_LEAVES + 2];
+    int l = from + 1;
+    compute_frame(t, b, l, frames[l]);
     for (;;) {
         GapFrame &f = frames[l];
         if (f.left > 0) {
             const int m = f.pos[--f.left];
-            a[l] = uint8_t(m);
+            after[l] = uint8_t(m);
             b[l] = b[m];
             b[m] = uint8_t(l);
-            a[b[l]] = uint8_t(l);
-            ++l;
-            enter(l);
+            if (l < depth) {
+                ++l;
+                compute_frame(t, b, l, frames[l]);
+                continue;
+            }
+            if (!emit(b)) return;
         } else {
-            --l;
-            if (l == 0) break;
-            b[a[l]] = b[l];
-            a[b[l]] = a[l];
+            b[l] = 0;
+            if (--l == from) return;
+        }
+        b[after[l]] = b[l];
+        b[l] = 0;
+    }
+}
+
+}  // namespace
+
+// The states are the descendants, in order, of the states at a shallower
+// depth: gone through once to count, and once more, those that the range
+// touches, to write.  Few states are kept from the first pass.
+LunnonStates::LunnonStates(const LunnonTables &t, int depth) : t_(t) {
+    constexpr size_t kKept = 32768;
+    depth_ = std::min(std::max(depth, 0), t.n);
+    split_ = std::max(0, std::min(depth_ - 4, t.n / 3 + 1));
+    uint8_t b[MF_MAX_LEAVES + 2] = {0};
+    const size_t rec = size_t(t.n) + 1;
+    expand_states(t_, b, 0, split_, [&](const uint8_t *c) {
+        roots_.insert(roots_.end(), c, c + rec);
+        return true;
+    });
+    const size_t roots = roots_.size() / rec;
+    first_.assign(roots + 1, 0);
+    each(0, roots, [&](size_t k, uint8_t *c, bool alone) {
+        uint64_t found = 0;
+        expand_states(t_, c, split_, depth_, [&](const uint8_t *s) {
+            ++found;
+            if (alone && kept_.size() < kKept * rec) kept_.insert(kept_.end(), s, s + rec);
+            return true;
+        });
+        first_[k + 1] = found;
+    });
+    for (size_t k = 0; k < roots; ++k) first_[k + 1] += first_[k];
+    if (kept_.size() != total() * rec) kept_.clear();
+}
+
+// run(k, b, alone) for roots lo <= k < hi, b a copy of root k: in order on
+// this thread (alone), and where more than 2.5 ms are left after 0.3 ms on all
+// the host's threads (6x6 to depth 18: 11.9 -> 2.3 ms).  A new thread may wait
+// for its core's next tick: 5x5 to depth 13, 0.4 ms on one, took 3.9 on 16.
+template <class F>
+void LunnonStates::each(size_t lo, size_t hi, F &&run) const {
+    const size_t rec = size_t(t_.n) + 1;
+    std::atomic<size_t> next{lo};
+    std::vector<std::thread> pool;
+    auto one = [&](size_t k, bool alone) {
+        uint8_t b[MF_MAX_LEAVES + 2] = {0};
+        std::memcpy(b, &roots_[k * rec], rec);
+        run(k, b, alone);
+    };
+    auto help = [&] {
+        for (size_t k; (k = next.fetch_add(1)) < hi;) one(k, false);
+    };
+    const double start = now_seconds();
+    for (size_t k; (k = next.fetch_add(1)) < hi;) {
+        one(k, pool.empty());
+        const double took = pool.empty() ? now_seconds() - start : 0;
+        if (took > 3e-4 && took * double(hi - k - 1) > 2.5e-3 * double(k + 1 - lo)) {
+            const size_t threads = std::min<size_t>({host_threads(), 16, (hi - k) / 4});
+            try {
+                for (size_t j = 1; j < threads; ++j) pool.emplace_back(help);
+            } catch (const std::system_error &) {  // no more threads: fewer do
+            }
         }
     }
-    return found;
+    for (auto &th : pool) th.join();
+}
+
+void LunnonStates::write(uint64_t first, uint64_t count, uint8_t *out, uint32_t stride) const {
+    const size_t rec = size_t(t_.n) + 1;
+    const uint64_t last = std::min(total(), first + count);
+    if (first >= last) return;
+    auto put = [&](uint64_t k, const uint8_t *b) {
+        uint8_t *to = out + (k - first) * stride;
+        std::memcpy(to, b, rec);
+        std::memset(to + rec, 0, stride - rec);
+    };
+    if (!kept_.empty()) {
+        for (uint64_t k = first; k < last; ++k) put(k, &kept_[k * rec]);
+        return;
+    }
+    const size_t lo = size_t(std::upper_bound(first_.begin(), first_.end(), first) - first_.begin()) - 1;
+    const size_t hi = size_t(std::lower_bound(first_.begin(), first_.end(), last) - first_.begin());
+    each(lo, hi, [&](size_t k, uint8_t *c, bool) {
+        uint64_t at = first_[k];
+        expand_states(t_, c, split_, depth_, [&](const uint8_t *b) {
+            if (at >= first) put(at, b);
+            return ++at < last;
+        });
+    });
+}
+
+uint64_t collect_lunnon_states(const LunnonTables &t, int depth, uint8_t *out, uint64_t cap,
+                               uint32_t stride, uint64_t first) {
+    const LunnonStates states(t, depth);
+    if (out) states.write(first, cap, out, stride);
+    return states.total();
 }
 
 // ---------------------------------------------------------------- sym ----
@@ -283,11 +367,6 @@ void sym_good_host_wide(const uint8_t *cycle, int i, const uint8_t *wide_edges, 
 namespace {
 
 constexpr int kMaxCentre = 25;  // 5 x 5 centre (experiments/9x9/sym_fold9.cpp:33)
-
-size_t host_threads() {
-    const unsigned hw = std::thread::hardware_concurrency();
-    return hw ? hw : 1;
-}
 
 // A centre cycle packed into one integer: cell v's successor (< 25, 5 bits)
 // at bits 5v..5v+4.  Equal cycles give equal keys.

@@ -900,9 +900,10 @@ int32_t mf_server_submit_lunnon(mf_server *s, const int32_t *dims, int32_t ndim,
         return MF_ERR_ARG;
     }
     const uint32_t stride = lunnon_state_stride(t.n);
-    const uint64_t total = collect_lunnon_states(t, depth, nullptr, 0, stride);
+    const LunnonStates list(t, depth);
+    const uint64_t total = list.total();
     std::vector<uint8_t> states(std::max<uint64_t>(total, 1) * stride);
-    collect_lunnon_states(t, depth, states.data(), total, stride);
+    list.write(0, total, states.data(), stride);
     auto r = std::make_shared<Request>();
     r->units.resize(total);
     for (uint64_t k = 0; k < total; ++k) {
