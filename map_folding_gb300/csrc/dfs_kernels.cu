@@ -127,26 +127,13 @@ __global__ void ring_init_kernel(unsigned long long *seq, unsigned long long cap
         seq[k] = k;
 }
 
-// Row counting (tail.cuh) of the persistent kernels.
-// Frames that make a level full, lanes at the row that start a count, and the
-// bookkeeping rounds that a count stands for (50,000 7x7 cases: 1,216 ms with
-// 16 / 24 / 16; fill 10: 1,312, fill 24: 1,257; roots 18: 1,294, roots 28:
-// 1,189; rounds 32: 1,232, rounds 8: 1,206).
-constexpr int kTailFill = 16;
-constexpr int kTailRoots = 28;
-constexpr uint32_t kTailRounds = 8;
-// Levels above the row from which a subtree may be handed out: below, an item
-// is a root or two and costs as much to pass on as to count (4x5 at
-// depth 12, with sharing within the warp: 310 us at 4, 244 at 6).
-constexpr int kRowSplit = 5;
-// ... and above the counted level where no row is counted by itself.
+// Split items of the persistent kernels start at least this high above the
+// counted level where no row is counted by itself.
 constexpr int kMinRingHeight = 6;
-constexpr int kRowShare = 1;  // the same for a piece shared within the warp
 // Idle lanes of a working warp that go for split items between bookkeepings:
 // every attempt stops the warp for two trips to L2 (500 7x7 cases: 30.8 ms with
 // 1, 29.1 with 16; 6x6: 135 and 131 ms).
 constexpr int kTakeLanes = 16;
-constexpr int kNoRow = 1 << 20;
 constexpr int kRowLevels = 4;  // Lunnon: levels to go, of a map with rows, from which they pay
 
 // Most cells of a list that the row count takes: all but two of a square's;
@@ -158,54 +145,13 @@ __host__ __device__ constexpr int tail_cells() {
 
 template <bool kSym, int TMAX>
 __host__ __device__ constexpr size_t tail_bytes(int tpb) {
-    if constexpr (TMAX > 0) return size_t(tpb / 32) * TailLayout<TMAX, tail_cells<kSym, TMAX>(), kTailFill>::kBytes;
+    if constexpr (TMAX > 0) return size_t(tpb / 32) * TailLayout<TMAX, tail_cells<kSym, TMAX>(), kTailFill, 5>::kBytes;
     else return 0;
 }
 
 template <bool kSym, int TMAX>
 __device__ __forceinline__ uint8_t *tail_of_warp(uint8_t *areas) {
     return areas + tail_bytes<kSym, TMAX>(int(threadIdx.x) & ~31);
-}
-
-// The pages of the last row of a square: the row's last cell is `last`, held
-// by last - 1 and by a cell of the row before.
-__device__ __forceinline__ TailPages sym_row_pages(const uint8_t *edge, int last) {
-    TailPages r{edge, edge, edge};
-    for (int p = 0; p < 4; ++p) {
-        const uint8_t *e = edge + p * kSymCells;
-        if (e[last] == last - 1) r.a1 = e;
-        else if (e[last] < last) r.b = e;
-        if (e[last - 1] == last - 2) r.a0 = e;
-    }
-    return r;
-}
-
-// Whether the arcs of the placed cells cross on no page: a page of k arcs has
-// k + 1 faces then and only then.  The row count takes that for granted; a
-// unit that a caller made up otherwise is searched by the list walk alone.
-template <class List>
-__device__ __forceinline__ bool pages_planar(const List &L, const uint8_t *edge, int placed) {
-    bool planar = placed <= kSymCells;
-#pragma unroll 1
-    for (int p = 0; p < 4; ++p) {
-        const uint8_t *e = edge + p * kSymCells;
-        uint64_t left = low_bits(placed);
-        int faces = 0, ends = 0;
-        while (left) {
-            const int g0 = low_bit(left);
-            int g = g0;
-            do {
-                left &= ~(1ULL << g);
-                const int c = L.get(g);
-                const int q = e[c];
-                ends += q < placed;
-                g = q < placed ? q : c;
-            } while (g != g0);
-            ++faces;
-        }
-        planar &= faces == ends / 2 + 1;
-    }
-    return planar;
 }
 
 struct SymSource {
@@ -278,7 +224,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
     if constexpr (TMAX > 0 && kSym) {
         if (sym.row > 0) {
             row_level = sym.last + 1 - sym.row;
-            pages = sym_row_pages(s_tables, sym.last);
+            pages = sym_row_pages(s_tables, sym.last, kSymCells);
         }
     }
 
@@ -461,7 +407,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                     S.base = root;
                     ok = list_valid(L, root);
                     if constexpr (TMAX > 0)
-                        row_level = sym.row > 0 && ok && pages_planar(L, s_tables, root)
+                        row_level = sym.row > 0 && ok && pages_planar(L, s_tables, kSymCells, root)
                                         ? sym.last + 1 - sym.row : kNoRow;
                 } else {
                     owner = pre_owner;
@@ -581,7 +527,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                         return kSym ? int(pages.b[last - e]) : last - e - row_len;
                     };
                     const int prev = eval > last + 1 - (kSym ? sym.row : row_len) ? eval - 1 : -1;
-                    ok = tail.setup(at, L, eval, K0, pages, w, prev, C, W, R, H);
+                    ok = tail.setup(L, eval, K0, pages, w, prev, C, W, R, H);
                     if (ok) {
                         counted = __popc(C) + (kSym ? 1 : 0);
                         if (!kSym) C &= ~(tail.word(RowTail::Y::kTop)[lane] & 1);

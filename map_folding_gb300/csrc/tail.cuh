@@ -16,8 +16,8 @@
 //            of gaps is a 32-bit mask and "after" is "greater".
 //   W[x]     the face of w_x on page b: where v_x may still go.
 //   P[x]     the gaps before w_x in list order (ones below a bit).
-//   planes   the faces of the gaps on the two row pages, as five bit planes of
-//            face numbers each: the gaps in the face of gap r are those whose
+//   planes   the faces of the gaps on the two row pages, as bit planes of face
+//            numbers, five each (six for 9x9): the gaps in the face of gap r are those whose
 //            plane bits equal r's.
 //
 // Placing v_t into gap r (bit b) draws the arc (w_t, v_t) on page b; every
@@ -47,9 +47,10 @@ namespace {
 // What a warp keeps in shared memory for its rows.  CELLS: the most cells a
 // root's list can have.  A level with FILL or more frames is run before a
 // shallower one, so no level ever holds more than FILL - 1 + 32.
-template <int TMAX, int CELLS, int FILL>
+// BITS: of a face number, enough for half as many faces as cells.
+template <int TMAX, int CELLS, int FILL, int BITS>
 struct TailLayout {
-    static_assert(CELLS <= 63 && FILL <= 32 && TMAX >= 2 && TMAX <= 8, "tail layout");
+    static_assert(CELLS <= (BITS == 5 ? 63 : 80) && FILL <= 32 && TMAX >= 2 && TMAX <= 8, "tail layout");
     static constexpr int kCap = FILL + 32;
     __host__ __device__ static constexpr int quads(int k) { return (3 + k + 3) / 4; }
     __host__ __device__ static constexpr int cap(int k) { return k == TMAX - 1 ? 32 : kCap; }
@@ -58,20 +59,18 @@ struct TailLayout {
         for (int j = 1; j < k; ++j) at += quads(j) * cap(j) * 16;
         return at;
     }
-    static constexpr int kPlane = 0;                         // 2 pages x 5 planes
-    static constexpr int kBefore = kPlane + 10 * 128;        // P of each level
+    static constexpr int kPlane = 0;                         // 2 pages x BITS planes
+    static constexpr int kBefore = kPlane + 2 * BITS * 128;  // P of each level
     static constexpr int kTop = kBefore + TMAX * 128;        // Lunnon: bit 0 the gap on the sentinel,
                                                              // << 8 the first level with an arc
     static constexpr int kAcc = kTop + 128;                  // leaves of each root
     static constexpr int kFrames = kAcc + 128;
-    // Scratch of the set-up, in the frames' place (they are empty then): per
-    // cell the face numbers before it and its place in the list, per place the
-    // face numbers after it; then the same of U's gaps only.
+    // Scratch of the set-up, in the frames' place (they are empty then): a word
+    // per cell (the face numbers before it, later also the gaps of U before it)
+    // and 16 words of face numbers per gap of U.
     static constexpr int kPre = kFrames;
-    static constexpr int kIds = kPre + (CELLS > 32 ? (CELLS + 1) / 2 * 2 : 32) * 64;
-    static constexpr int kPos = kIds + CELLS * 64;
-    static constexpr int kScratchEnd = kPos + CELLS * 32;
-    static constexpr int kGapIds = kPre;  // over the cells' face numbers: 16 words a lane
+    static constexpr int kGapIds = kPre + CELLS * 128;
+    static constexpr int kScratchEnd = kGapIds + 16 * 128;
     static constexpr int kEnd = frames(TMAX);
     static constexpr int kBytes = ((kEnd > kScratchEnd ? kEnd : kScratchEnd) + 127) / 128 * 128;
 };
@@ -94,9 +93,9 @@ struct TailPages {
 // kSym: a square's side, always of TMAX cells; else rows of a Lunnon map, of up
 // to TMAX leaves (a longer row starts inside), whose gap on the sentinel counts
 // as a node and is not searched.
-template <bool kSym, int TMAX, int CELLS, int FILL>
+template <bool kSym, int TMAX, int CELLS, int FILL, int BITS = 5>
 struct Tail {
-    using Y = TailLayout<TMAX, CELLS, FILL>;
+    using Y = TailLayout<TMAX, CELLS, FILL, BITS>;
     static constexpr int kRow = TMAX;
     uint8_t *area;
     int lane;
@@ -108,94 +107,95 @@ struct Tail {
     // Bit of h(ex, es): the half of v_es's gap that the pending level ex keeps.
     __device__ static constexpr int hbit(int ex, int es) { return es * (es - 1) / 2 - 1 + ex; }
 
-    // Clear the set-up's scratch for lists of `placed` cells (all lanes call).
+    // Clear the set-up's scratch (all lanes call).
     __device__ __forceinline__ void prepare_setup() const {
         uint4 *pre = reinterpret_cast<uint4 *>(area + Y::kPre);
 #pragma unroll
-        for (int k = 0; k < (Y::kIds - Y::kPre) / 16; k += 32)
-            if (k + lane < (Y::kIds - Y::kPre) / 16) pre[k + lane] = make_uint4(~0u, ~0u, ~0u, ~0u);
+        for (int k = 0; k < CELLS * 8; k += 32)
+            if (k + lane < CELLS * 8) pre[k + lane] = make_uint4(~0u, ~0u, ~0u, ~0u);
         __syncwarp();
     }
 
     // Write down a root: the list L of `placed` cells, row levels K0 .. 0 to
     // come, w(e) the row-before neighbour of level e's cell and prev the cell
-    // before the first (< 0: none, the row starts here).  The lanes in `lanes`
-    // call together.  Returns false if the root has more than 31 gaps.  Fills the root's tables and hands back the frame
+    // before the first (< 0: none, the row starts here).  Returns false if it
+    // has more than 31 gaps.  Fills the root's tables and hands back the frame
     // in registers.
     //
     // One pass over the list in order, with no data-dependent branch so that
     // all lanes stay together: going past the first end of an arc enters a new
     // face, past the second end returns to the face before the first.  (Walking
     // each face by itself took 8 times as long, the lanes' walks being of
-    // different lengths.)  The face numbers of the gaps in U, one 16-bit word
-    // per gap, are then turned into planes by a 16 x 16 bit transposition.
+    // different lengths.)  A second pass numbers the gaps of U; their face
+    // numbers are then turned into planes by a 16 x 16 bit transposition.
     template <class List, class WOf>
-    __device__ __forceinline__ bool setup(unsigned lanes, const List &L, int placed, int K0,
-                                          const TailPages &pg, WOf &&w, int prev, uint32_t &C, uint32_t (&W)[TMAX],
+    __device__ __forceinline__ bool setup(const List &L, int placed, int K0, const TailPages &pg,
+                                          WOf &&w, int prev, uint32_t &C, uint32_t (&W)[TMAX],
                                           uint32_t &R, uint32_t &H) const {
-        uint16_t *pre = reinterpret_cast<uint16_t *>(area + Y::kPre) + lane;
-        uint16_t *ids = reinterpret_cast<uint16_t *>(area + Y::kIds) + lane;
-        uint8_t *pos = area + Y::kPos + lane;
+        constexpr uint32_t kField = (1u << BITS) - 1;
+        constexpr uint32_t kIds = (1u << (3 * BITS)) - 1;
+        uint32_t *pre = word(Y::kPre) + lane;
         // Face numbers of the gap at hand and the highest given out: page b in
-        // bits 0-4, a0 in 5-9, a1 in 10-14.
+        // the low field, then a0, a1.
         uint32_t f = 0, top = 0;
         int c = 0;
 #pragma unroll 1
         for (int i = 0; i < placed; ++i) {
-            pre[c * 32] = uint16_t(f);
-            pos[c * 32] = uint8_t(i);
+            pre[c * 32] = f | uint32_t(i) << 20;
             const int after = L.get(c);
             const int q0 = pg.b[c], q1 = pg.a0[c], q2 = pg.a1[c];
             // No placed partner: c's own entry, which changes nothing.
             const uint32_t v0 = pre[(q0 < placed ? q0 : c) * 32];
             const uint32_t v1 = pre[(q1 < placed ? q1 : c) * 32];
             const uint32_t v2 = pre[(q2 < placed ? q2 : c) * 32];
-            if (v0 == 0xffffu) top += 1u;
-            if (v1 == 0xffffu) top += 1u << 5;
-            if (v2 == 0xffffu) top += 1u << 10;
-            f = ((v0 == 0xffffu ? top : v0) & 0x001fu) | ((v1 == 0xffffu ? top : v1) & 0x03e0u) |
-                ((v2 == 0xffffu ? top : v2) & 0x7c00u);
-            ids[i * 32] = uint16_t(f);
+            if (v0 == ~0u) top += 1u;
+            if (v1 == ~0u) top += 1u << BITS;
+            if (v2 == ~0u) top += 1u << (2 * BITS);
+            f = ((v0 == ~0u ? top : v0) & kField) | ((v1 == ~0u ? top : v1) & (kField << BITS)) |
+                ((v2 == ~0u ? top : v2) & (kField << (2 * BITS)));
             c = after;
         }
         // Not one cycle (cell 0 met again before the end): left to the list walk.
-        const bool cycle = c == 0 && pos[0] == 0;
+        if (c != 0 || pre[0] >> 20 != 0) return false;
         // The faces of the w's on page b (a w has no arc there, so its gap is
         // in the face before it).
         uint32_t fw[TMAX];
-        int at[TMAX];
-        uint32_t set = 0;
+        uint64_t set = 0;
 #pragma unroll
         for (int e = 0; e < TMAX; ++e) {
             fw[e] = 0;
-            at[e] = 0;
             if (e <= K0) {
-                const int x = w(e);
-                fw[e] = pre[x * 32] & 31u;
-                at[e] = pos[x * 32];
-                set |= 1u << fw[e];
+                fw[e] = pre[w(e) * 32] & kField;
+                set |= 1ULL << fw[e];
             }
         }
         const uint32_t fprev = prev >= 0 ? pre[prev * 32] : 0;
-        __syncwarp(lanes);  // the gap ids go over other lanes' `pre`
-        // U in list order.
-        uint64_t places = 0;
+        // U in list order; each cell learns how many of its gaps come before.
         int gaps = 0;
+        uint32_t first_in = 0, plane16 = 0, plane17 = 0;
         uint16_t *gap_ids = reinterpret_cast<uint16_t *>(area + Y::kGapIds) + 2 * lane;
-#pragma unroll 2
+#pragma unroll 1
         for (int i = 0; i < placed; ++i) {
-            const uint32_t v = ids[i * 32];
-            const bool in = (set >> (v & 31)) & 1;
+            reinterpret_cast<uint8_t *>(pre + c * 32)[3] = uint8_t(gaps);
+            c = L.get(c);
+            const uint32_t v = pre[c * 32] & kIds;
+            const bool in = BITS == 5 ? (uint32_t(set) >> (v & kField)) & 1 : (set >> (v & kField)) & 1;
             if (in && gaps < 32) {
                 gap_ids[(gaps & 15) * 64 + (gaps >> 4)] = uint16_t(v);
-                places |= 1ULL << i;
+                if (BITS == 6) {
+                    plane16 |= ((v >> 16) & 1) << gaps;
+                    plane17 |= ((v >> 17) & 1) << gaps;
+                }
             }
+            if (!kSym && i == 0) first_in = in;
             gaps += in;
         }
-        if (!cycle || gaps > 31) return false;
-        uint32_t a[16];
+        if (gaps > 31) return false;
+        uint32_t a[18];
 #pragma unroll
         for (int j = 0; j < 16; ++j) a[j] = word(Y::kGapIds)[j * 32 + lane];
+        a[16] = plane16;
+        a[17] = plane17;
 #pragma unroll
         for (int t = 8; t >= 1; t >>= 1) {
             const uint32_t m = t == 8 ? 0x00ff00ffu : t == 4 ? 0x0f0f0f0fu
@@ -209,20 +209,19 @@ struct Tail {
                 }
         }
 #pragma unroll
-        for (int j = 0; j < 10; ++j) word(Y::kPlane)[j * 32 + lane] = a[5 + j];
+        for (int j = 0; j < 2 * BITS; ++j) word(Y::kPlane)[j * 32 + lane] = a[BITS + j];
         const uint32_t all = (1u << gaps) - 1;
         C = 0;
 #pragma unroll
         for (int e = TMAX - 1; e >= 0; --e) {
             uint32_t m = all;
 #pragma unroll
-            for (int j = 0; j < 5; ++j) m &= (fw[e] >> j) & 1 ? a[j] : ~a[j];
+            for (int j = 0; j < BITS; ++j) m &= (fw[e] >> j) & 1 ? a[j] : ~a[j];
             W[e] = e <= K0 ? m : 0;
             if (e == K0) C = m;
-            word(Y::kBefore)[e * 32 + lane] = (1u << __popcll(places & low_bits(at[e]))) - 1;
+            word(Y::kBefore)[e * 32 + lane] = e <= K0 ? (1u << (pre[w(e) * 32] >> 24)) - 1 : 0;
         }
-        if (!kSym)
-            word(Y::kTop)[lane] = uint32_t(places & 1) | uint32_t(prev >= 0 ? TMAX : K0) << 8;
+        if (!kSym) word(Y::kTop)[lane] = first_in | uint32_t(prev >= 0 ? TMAX : K0) << 8;
         R = 0;
         H = uint32_t(lane) << 27;
         if (prev >= 0) {
@@ -230,15 +229,15 @@ struct Tail {
             // arc, and it stands in for all earlier picks (an arc between two
             // equal picks encloses nothing).
             const bool odd = (K0 + 1) & 1;
-            const uint32_t fp = odd ? fprev >> 10 : fprev >> 5;
+            const uint32_t fp = odd ? fprev >> (2 * BITS) : fprev >> BITS;
             uint32_t m = ~0u;
 #pragma unroll
-            for (int j = 0; j < 5; ++j) {
-                const uint32_t plane = word(Y::kPlane)[((odd ? 5 : 0) + j) * 32 + lane];
+            for (int j = 0; j < BITS; ++j) {
+                const uint32_t plane = word(Y::kPlane)[((odd ? BITS : 0) + j) * 32 + lane];
                 m &= (fp >> j) & 1 ? plane : ~plane;
             }
             C &= m;
-            const uint32_t before = uint32_t(__popcll(places & low_bits(pos[prev * 32])));
+            const uint32_t before = pre[prev * 32] >> 24;
 #pragma unroll
             for (int j = 0; j < 6; ++j) R |= before << (5 * j);
             H |= (~0u << hbit(0, K0 + 1)) & 0x07ffffffu;
@@ -352,10 +351,10 @@ struct Tail {
                     const uint32_t info = kSym ? 0 : word(Y::kTop)[slot];
                     const int r = 31 - __clz(int(bt));
                     const uint32_t *before = word(Y::kBefore) + slot;
-                    const uint32_t *plane = word(Y::kPlane) + (K & 1) * 160 + slot;
+                    const uint32_t *plane = word(Y::kPlane) + (K & 1) * 32 * BITS + slot;
                     uint32_t face = ~0u;
 #pragma unroll
-                    for (int j = 0; j < 5; ++j) {
+                    for (int j = 0; j < BITS; ++j) {
                         const uint32_t p = plane[j * 32];
                         face &= p & bt ? p : ~p;
                     }
@@ -414,6 +413,64 @@ struct Tail {
         }
     }
 };
+
+// Row counting of the persistent kernels.  Frames that make a level full, lanes
+// at the row that start a count, and the bookkeeping rounds that a count
+// stands for (50,000 7x7 cases: 1,216 ms with 16 / 24 / 16; fill 10: 1,312,
+// fill 24: 1,257; roots 18: 1,294, roots 28: 1,189; rounds 32: 1,232, rounds 8:
+// 1,206).
+constexpr int kTailFill = 16;
+constexpr int kTailRoots = 28;
+constexpr uint32_t kTailRounds = 8;
+// Levels above the row from which a subtree may be handed out: below, an item
+// is a root or two and costs as much to pass on as to count (4x5 at depth 12,
+// with sharing within the warp: 310 us at 4, 244 at 6).
+constexpr int kRowSplit = 5;
+constexpr int kRowShare = 1;  // the same for a piece shared within the warp
+constexpr int kNoRow = 1 << 20;
+
+// The pages of the last row of a square: the row's last cell is `last`, held
+// by last - 1 and by a cell of the row before.  `stride` cells per page.
+__device__ __forceinline__ TailPages sym_row_pages(const uint8_t *edge, int last, int stride) {
+    TailPages r{edge, edge, edge};
+    for (int p = 0; p < 4; ++p) {
+        const uint8_t *e = edge + p * stride;
+        if (e[last] == last - 1) r.a1 = e;
+        else if (e[last] < last) r.b = e;
+        if (e[last - 1] == last - 2) r.a0 = e;
+    }
+    return r;
+}
+
+// Whether the arcs of the placed cells cross on no page: a page of k arcs has
+// k + 1 faces then and only then.  The row count takes that for granted; a
+// unit that a caller made up otherwise is searched by the list walk alone.
+template <class List>
+__device__ __forceinline__ bool pages_planar(const List &L, const uint8_t *edge, int stride,
+                                             int placed) {
+    bool planar = true;
+#pragma unroll 1
+    for (int p = 0; p < 4; ++p) {
+        const uint8_t *e = edge + p * stride;
+        uint64_t seen[2] = {0, 0};
+        int faces = 0, ends = 0;
+        for (int g0 = 0; g0 < placed; ++g0) {
+            if (((g0 < 64 ? seen[0] : seen[1]) >> (g0 & 63)) & 1) continue;
+            int g = g0;
+            do {
+                if (g < 64) seen[0] |= 1ULL << g;
+                else seen[1] |= 1ULL << (g & 63);
+                const int c = L.get(g);
+                const int q = e[c];
+                ends += q < placed;
+                g = q < placed ? q : c;
+            } while (g != g0);
+            ++faces;
+        }
+        planar &= faces == ends / 2 + 1;
+    }
+    return planar;
+}
 
 }  // namespace
 }  // namespace mf

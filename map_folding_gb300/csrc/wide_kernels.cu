@@ -14,6 +14,7 @@
 
 #include "dfs_core.cuh"
 #include "engine.hpp"
+#include "tail.cuh"
 
 namespace mf {
 namespace {
@@ -50,7 +51,7 @@ constexpr size_t kWideTables = 1280;
 static_assert(kWidePages + 8 * kWideCells + kWideCells <= kWideTables, "wide table layout");
 constexpr int kWideWords = kWideCells / 4;  // list words per lane
 constexpr int kWideRecordWords = 32;        // 128-byte split records
-static_assert(kWideWords + 4 + 2 <= kWideRecordWords, "wide record layout");
+static_assert(kWideWords + 4 + 3 <= kWideRecordWords, "wide record layout");
 
 template <int TPB>
 __device__ __forceinline__ void stage_wide_tables(uint8_t *smem, const uint8_t *__restrict__ edges) {
@@ -140,18 +141,52 @@ struct StackW {
     __device__ __forceinline__ void set_pick(int lvl, int j) const { chosen.put(lvl - base, j); }
 };
 
+// The same in local memory, for the kernel that counts the last row by itself:
+// it needs the shared memory for that, and its list search is a few nodes in a
+// hundred.
+template <int LEVELS>
+struct LocalStackW {
+    uint64_t lo[LEVELS], hi[kWideHiRows];
+    uint8_t chosen[LEVELS];
+    int base;
+    __device__ __forceinline__ Mask128 get(int lvl) const {
+        return Mask128{lo[lvl - base], lvl > 64 ? hi[lvl - 65] : 0ULL};
+    }
+    __device__ __forceinline__ void set(int lvl, const Mask128 &v) {
+        lo[lvl - base] = v.lo;
+        if (lvl > 64) hi[lvl - 65] = v.hi;
+    }
+    __device__ __forceinline__ int pick(int lvl) const { return chosen[lvl - base]; }
+    __device__ __forceinline__ void set_pick(int lvl, int j) { chosen[lvl - base] = uint8_t(j); }
+};
+
+// Row counting on the 9x9 board: its last eight cells (the layout's most; a
+// row of nine starts with the list walk).
+constexpr int kWideRow = 8;
+constexpr int kWideTailCells = 79;
+using WideTail = Tail<true, kWideRow, kWideTailCells, kTailFill, 6>;
+
+template <int TPB, int LEVELS, bool kRow>
+struct WideStack {
+    using type = StackW<TPB, LEVELS>;
+};
+template <int TPB, int LEVELS>
+struct WideStack<TPB, LEVELS, true> {
+    using type = LocalStackW<LEVELS>;
+};
+
 template <int TPB, int LEVELS>
 struct CarveW {
     static constexpr size_t kList = size_t(kWideWords) * 4 * TPB;
     static constexpr size_t kMask = size_t(LEVELS + kWideHiRows) * 8 * TPB;
     static constexpr size_t kPick = size_t((LEVELS + 3) / 4) * 4 * TPB;
     static constexpr size_t kBytes = kWideTables + kList + kMask + kPick;
+    static constexpr size_t kRowBytes = kWideTables + kList + TPB / 32 * WideTail::Y::kBytes;
 };
 
 // advance of dfs_core.cuh with 128-bit masks (a taken split item starts here).
-template <int TPB, int LEVELS>
-__device__ __forceinline__ int advance_w(const List<TPB> &L, const StackW<TPB, LEVELS> &S, int &lvl,
-                                         int root) {
+template <class List, class Stk>
+__device__ __forceinline__ int advance_w(const List &L, Stk &S, int &lvl, int root) {
     for (;;) {
         const Mask128 cur = S.get(lvl);
         if (w_zero(cur)) {
@@ -172,10 +207,10 @@ __device__ __forceinline__ int advance_w(const List<TPB> &L, const StackW<TPB, L
 // apply_advance of dfs_core.cuh with 128-bit masks: consume level eval's
 // mask g (handed over in registers) and move to the next node; -1 when the
 // unit's subtree is exhausted.
-template <int TPB, int LEVELS>
-__device__ __forceinline__ int apply_advance_w(const List<TPB> &L, const StackW<TPB, LEVELS> &S,
-                                               int &lvl, int eval, int root, int last, bool fresh,
-                                               const Mask128 &g, unsigned long long &leaves) {
+template <class List, class Stk>
+__device__ __forceinline__ int apply_advance_w(const List &L, Stk &S, int &lvl, int eval, int root,
+                                               int last, bool fresh, const Mask128 &g,
+                                               unsigned long long &leaves) {
     Mask128 cur;
     if (eval == last) {
         leaves += w_popc(g);
@@ -235,9 +270,11 @@ __device__ __forceinline__ void wide_put(uint4 *slots, const Queue &Q, unsigned 
 // 128-bit masks: initial units by a warp-aggregated atomicAdd, lockstep
 // rounds, bookkeeping every `period` rounds (idle-lane report, donation of
 // the shallowest untried siblings while lanes wait), split items taken by
-// idle lanes, and the same leaving rule.  Split record: list words
-// 0..kWideWords-1, owner, untried mask (4 words), level.
-template <int TPB, int LEVELS>
+// Split record: list words 0..kWideWords-1, owner, untried mask (4 words),
+// level, whether the row may be counted on masks.
+// idle lanes, and the same leaving rule; lanes of a warp share as there.  With
+// kRow the last cells of the 9x9 row are counted on masks (tail.cuh).
+template <int TPB, int LEVELS, bool kRow>
 __global__ void __launch_bounds__(TPB)
     sym_wide_kernel(const uint8_t *__restrict__ edges, int start_i, int last,
                     const uint8_t *__restrict__ cycles, uint32_t record_bytes, unsigned long long num,
@@ -248,15 +285,26 @@ __global__ void __launch_bounds__(TPB)
     __syncthreads();
     using C = CarveW<TPB, LEVELS>;
     const SymRulesW R = wide_rules(smem);
-    const List<TPB> L{smem + kWideTables + 4 * threadIdx.x};
-    StackW<TPB, LEVELS> S;
-    S.lo = reinterpret_cast<uint64_t *>(smem + kWideTables + C::kList) + threadIdx.x;
-    S.chosen = List<TPB>{smem + kWideTables + C::kList + C::kMask + 4 * threadIdx.x};
+    const List<TPB> L = List<TPB>::at(smem + kWideTables, kWideCells);
+    typename WideStack<TPB, LEVELS, kRow>::type S;
+    if constexpr (!kRow) {
+        S.lo = reinterpret_cast<uint64_t *>(smem + kWideTables + C::kList) + threadIdx.x;
+        S.chosen = List<TPB>::at(smem + kWideTables + C::kList + C::kMask, (LEVELS + 3) / 4 * 4);
+    }
     S.base = start_i;
 
     const int lane = threadIdx.x & 31;
+    WideTail tail;
+    tail.area = smem + kWideTables + C::kList + threadIdx.x / 32 * WideTail::Y::kBytes;
+    tail.lane = lane;
+    TailPages pages{};
+    if constexpr (kRow) pages = sym_row_pages(smem, last, kWideCells);
+    const int row_first = last + 1 - kWideRow;  // first level of the counted row
+    int row_level = kNoRow;                     // ... of the unit at hand
+    bool by_walk = false, whole = true, share_miss = false;
     const unsigned lt_mask = (1u << lane) - 1u;
-    constexpr int kOwner = kWideWords, kMaskW = kWideWords + 1, kRoot = kWideWords + 5;
+    constexpr int kOwner = kWideWords, kMaskW = kWideWords + 1, kRoot = kWideWords + 5,
+                  kRowOk = kWideWords + 6;
     bool busy = false, fresh = false, init_left = true;
     int lvl = start_i, root = start_i, eval = start_i;
     uint32_t owner = 0;
@@ -268,7 +316,7 @@ __global__ void __launch_bounds__(TPB)
     auto flush = [&]() {
         if (leaves) atomicAdd(counts + owner, leaves);
         leaves = 0;
-        ++finished;
+        if (whole) ++finished;
     };
 
     auto take_splits = [&](unsigned need) -> bool {
@@ -289,20 +337,28 @@ __global__ void __launch_bounds__(TPB)
                                 uint64_t(w[kMaskW + 2]) | (uint64_t(w[kMaskW + 3]) << 32)});
             eval = advance_w(L, S, lvl, root);  // an item's mask is never empty
             fresh = false;
+            whole = true;
+            by_walk = false;
+            if (kRow) row_level = w[kRowOk] ? row_first : kNoRow;
             busy = eval >= 0;
             if (!busy) ++finished;
         }
         return got < want;
     };
 
+    // The shallowest level with untried siblings, and those.
+    auto shallowest = [&](int &s) -> Mask128 {
+        s = root;
+        if (!busy || fresh) return Mask128{0, 0};
+        while (s < lvl && w_zero(S.get(s))) ++s;
+        return S.get(s);
+    };
+
     auto donate = [&]() {
         int s = root;
-        Mask128 m{0, 0};
-        if (busy && !fresh) {
-            while (s < lvl && w_zero(S.get(s))) ++s;
-            m = S.get(s);
-        }
-        const bool can = busy && !fresh && !w_zero(m) && last - s >= kMinSplitHeight;
+        const Mask128 m = shallowest(s);
+        const bool can = !w_zero(m) && (row_level != kNoRow ? row_level - s >= kRowSplit
+                                                            : last - s >= kMinSplitHeight);
         const unsigned donors = __ballot_sync(kFull, can);
         if (!donors) return;
         unsigned long long first = 0;
@@ -321,6 +377,7 @@ __global__ void __launch_bounds__(TPB)
         w[kMaskW + 2] = uint32_t(m.hi);
         w[kMaskW + 3] = uint32_t(m.hi >> 32);
         w[kRoot] = uint32_t(s);
+        w[kRowOk] = row_level != kNoRow;
         for (int l = s; l <= lvl; ++l) {
             const int j = S.pick(l);
             L.put(l, L.get(j));
@@ -328,6 +385,51 @@ __global__ void __launch_bounds__(TPB)
         }
         S.set(s, Mask128{0, 0});
         wide_put(slots, Q, first + rank, w);
+    };
+
+    // share_in_warp of dfs_core.cuh with 128-bit masks and separate picks.
+    auto share = [&](unsigned idle) -> bool {
+        int s = root;
+        const Mask128 m = shallowest(s);
+        const int floor = row_level != kNoRow ? row_level - kRowShare : last - kMinShareHeight;
+        const unsigned donors = shallowest_lanes(!w_zero(m) && s <= floor, s, __popc(idle));
+        const int n = __popc(donors);
+        if (n == 0) return false;
+        const bool give = (donors >> lane) & 1u;
+        const int rank = __popc(idle & lt_mask);
+        const bool take = ((idle >> lane) & 1u) && rank < n;
+        const int from = take ? nth_bit(donors, rank) : lane;
+        if (give)
+            for (int l = lvl; l >= s; --l) L.put(S.pick(l), L.get(l));
+        __syncwarp();
+        const int level = __shfl_sync(kFull, s, from);
+        const Mask128 mask{__shfl_sync(kFull, m.lo, from), __shfl_sync(kFull, m.hi, from)};
+        const uint32_t whose = __shfl_sync(kFull, owner, from);
+        const int its_row = __shfl_sync(kFull, row_level, from);
+        if (take) {
+            const List<TPB> theirs{L.base + 4 * (from - lane)};
+            for (int j = 0; j < level; ++j) L.put(j, theirs.get(j));
+            owner = whose;
+            row_level = its_row;
+            root = level;
+            lvl = level;
+            S.set(root, mask);
+            eval = advance_w(L, S, lvl, root);
+            whole = false;
+            fresh = false;
+            by_walk = false;
+            busy = true;
+        }
+        __syncwarp();
+        if (give) {
+            for (int l = s; l <= lvl; ++l) {
+                const int j = S.pick(l);
+                L.put(l, L.get(j));
+                L.put(j, l);
+            }
+            S.set(s, Mask128{0, 0});
+        }
+        return true;
     };
 
     for (;;) {
@@ -358,7 +460,13 @@ __global__ void __launch_bounds__(TPB)
                     owner = uint32_t(k);
                     root = start_i;
                     ++started;
-                    if (!list_valid(L, start_i)) {
+                    whole = true;
+                    by_walk = false;
+                    const bool ok = list_valid(L, start_i);
+                    if (kRow)
+                        row_level = ok && pages_planar(L, smem, kWideCells, start_i) ? row_first
+                                                                                     : kNoRow;
+                    if (!ok) {
                         atomicExch(&Q.hdr->error, kErrMalformed);
                         ++finished;
                     } else if (start_i > last) {
@@ -375,6 +483,8 @@ __global__ void __launch_bounds__(TPB)
                 }
             }
         }
+        const unsigned unfed = __ballot_sync(kFull, !busy && !init_left);
+        if (__popc(unfed) >= kShareLanes && unfed != kFull && !share_miss) share_miss = !share(unfed);
         if (ring_hint) {
             const unsigned need = __ballot_sync(kFull, !busy && !init_left);
             if (need && take_splits(need)) ring_hint = false;
@@ -413,13 +523,45 @@ __global__ void __launch_bounds__(TPB)
         }
         idle_rounds = 0;
         nap = 256;
-        if (busy) {
+        auto at_row = [&]() { return kRow && busy && eval >= row_level && eval < last && !by_walk; };
+        if (busy && !at_row()) {
             const Mask128 g = R.gaps(L, eval, nodes);
+            by_walk = false;
             eval = apply_advance_w(L, S, lvl, eval, root, last, fresh, g, leaves);
             fresh = false;
             if (eval < 0) {
                 flush();
                 busy = false;
+            }
+        }
+        if constexpr (kRow) {
+            const bool here = at_row();
+            const unsigned at = __ballot_sync(kFull, here);
+            if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
+                uint32_t W[WideTail::kRow] = {};
+                uint32_t c = 0, r = 0, h = 0, counted = 0;
+                bool ok = false;
+                tail.prepare_setup();
+                if (here) {
+                    auto w = [&](int e) -> int { return pages.b[last - e]; };
+                    ok = tail.setup(L, eval, last - eval, pages, w, eval - 1, c, W, r, h);
+                    if (ok) counted = __popc(c) + 1;
+                    else by_walk = true;
+                }
+                tail.enqueue_roots(ok, last - eval, c, W, r, h);
+                tail.drain(counted);
+                nodes += counted;
+                if (ok) {
+                    leaves += tail.word(WideTail::Y::kAcc)[lane];
+                    eval = apply_advance_w(L, S, lvl, eval, root, last, fresh, Mask128{0, 0}, leaves);
+                    fresh = false;
+                    if (eval < 0) {
+                        flush();
+                        busy = false;
+                    }
+                }
+                __syncwarp();
+                round += kTailRounds;
             }
         }
         if (!bookkeeping) continue;
@@ -443,6 +585,7 @@ __global__ void __launch_bounds__(TPB)
         }
         want = __shfl_sync(kFull, want, 0);
         ring_hint = __shfl_sync(kFull, queued, 0) > 0;
+        share_miss = false;
         if (want > 0) donate();
     }
 
@@ -464,9 +607,7 @@ __global__ void wide_ring_init(unsigned long long *seq, unsigned long long capac
         seq[k] = k;
 }
 
-constexpr int kWideTPB = 64;
-
-template <int LEVELS>
+template <int kWideTPB, int LEVELS, bool kRow>
 cudaError_t launch_wide_levels(const uint8_t *d_edges, int start_i, int last, const uint8_t *d_cycles,
                                uint32_t record_bytes, uint64_t num, uint64_t *d_counts, uint64_t *d_nodes, const Queue &Q,
                                uint4 *slots, const BatchKnobs &knobs, cudaStream_t stream) {
@@ -475,24 +616,25 @@ cudaError_t launch_wide_levels(const uint8_t *d_edges, int start_i, int last, co
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return e;
-    constexpr size_t smem = CarveW<kWideTPB, LEVELS>::kBytes;
+    constexpr size_t smem =
+        kRow ? CarveW<kWideTPB, LEVELS>::kRowBytes : CarveW<kWideTPB, LEVELS>::kBytes;
     {
         std::lock_guard<std::mutex> lock(mu);
         if (dev < 0 || dev >= 16) return cudaErrorInvalidDevice;
         if (!raised[dev]) {
-            e = cudaFuncSetAttribute(sym_wide_kernel<kWideTPB, LEVELS>,
+            e = cudaFuncSetAttribute(sym_wide_kernel<kWideTPB, LEVELS, kRow>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem));
             if (e != cudaSuccess) return e;
             raised[dev] = true;
         }
     }
     int fit = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, sym_wide_kernel<kWideTPB, LEVELS>,
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, sym_wide_kernel<kWideTPB, LEVELS, kRow>,
                                                       kWideTPB, smem);
     if (e != cudaSuccess) return e;
     if (fit < 1) return cudaErrorInvalidConfiguration;
     if (knobs.blocks_per_sm > 0 && int(knobs.blocks_per_sm) < fit) fit = int(knobs.blocks_per_sm);
-    sym_wide_kernel<kWideTPB, LEVELS><<<unsigned(device_sm_count() * fit), kWideTPB, smem, stream>>>(
+    sym_wide_kernel<kWideTPB, LEVELS, kRow><<<unsigned(device_sm_count() * fit), kWideTPB, smem, stream>>>(
         d_edges, start_i, last, d_cycles, record_bytes, num,
         reinterpret_cast<unsigned long long *>(d_counts),
         reinterpret_cast<unsigned long long *>(d_nodes), Q, slots, knobs.node_budget,
@@ -532,12 +674,18 @@ cudaError_t launch_sym_wide(const uint8_t *d_wide_edges, int start_i, int stop_i
     if ((record_bytes != kSymCells && record_bytes != kWideCells) || start_i > int(record_bytes) ||
         stop_i > 66 + kWideHiRows || stop_i > kWideCells)
         return cudaErrorInvalidValue;
+    // The whole 9x9 row is nearly all of the search; near its end there is
+    // nothing above it to search by list.
+    if (stop_i == 81 && start_i <= stop_i - kWideRow && levels <= 56)
+        return launch_wide_levels<128, 56, true>(d_wide_edges, start_i, stop_i - 1, d_cycles,
+                                                 record_bytes, num, d_counts, d_nodes, Q, slots,
+                                                 knobs, stream);
     if (levels <= 40)
-        return launch_wide_levels<40>(d_wide_edges, start_i, stop_i - 1, d_cycles, record_bytes, num,
+        return launch_wide_levels<64, 40, false>(d_wide_edges, start_i, stop_i - 1, d_cycles, record_bytes, num,
                                       d_counts,
                                       d_nodes, Q, slots, knobs, stream);
     if (levels <= 56)
-        return launch_wide_levels<56>(d_wide_edges, start_i, stop_i - 1, d_cycles, record_bytes, num,
+        return launch_wide_levels<64, 56, false>(d_wide_edges, start_i, stop_i - 1, d_cycles, record_bytes, num,
                                       d_counts,
                                       d_nodes, Q, slots, knobs, stream);
     return cudaErrorInvalidValue;  // deeper searches need a deeper expansion first
