@@ -165,15 +165,51 @@ const uint8_t *device_wide_edges(int n) {
     return g_wide_edges[dev][n];
 }
 
+// Timing events of each device, given back after a call: making and destroying
+// six of them took a sixth of a small map's call.
+struct EventPool {
+    static constexpr size_t kMost = 64;
+    std::mutex mu;
+    std::vector<cudaEvent_t> free[16];
+    cudaEvent_t take(int dev) {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (dev >= 0 && dev < 16 && !free[dev].empty()) {
+                cudaEvent_t e = free[dev].back();
+                free[dev].pop_back();
+                return e;
+            }
+        }
+        cudaEvent_t e = nullptr;
+        cudaEventCreate(&e);
+        return e;
+    }
+    void give(int dev, cudaEvent_t e) {
+        {
+            std::lock_guard<std::mutex> lock(mu);
+            if (e && dev >= 0 && dev < 16 && free[dev].size() < kMost) {
+                free[dev].push_back(e);
+                return;
+            }
+        }
+        if (e) cudaEventDestroy(e);
+    }
+};
+EventPool g_events;
+
 struct Timer {
+    int dev = -1;
     cudaEvent_t a = nullptr, b = nullptr;
     Timer() {
-        cudaEventCreate(&a);
-        cudaEventCreate(&b);
+        cudaGetDevice(&dev);
+        a = g_events.take(dev);
+        b = g_events.take(dev);
     }
+    Timer(const Timer &) = delete;
+    Timer &operator=(const Timer &) = delete;
     ~Timer() {
-        cudaEventDestroy(a);
-        cudaEventDestroy(b);
+        g_events.give(dev, a);
+        g_events.give(dev, b);
     }
     double seconds() {
         float ms = 0;
@@ -183,6 +219,10 @@ struct Timer {
 };
 
 using u128 = unsigned __int128;
+
+// Bytes of `n` counters ahead of a workspace (which is 256-byte aligned): the
+// counts and the run header behind them come back in one copy.
+size_t counter_bytes(size_t n) { return (n * sizeof(uint64_t) + 255) / 256 * 256; }
 
 }  // namespace
 }  // namespace mf
@@ -429,8 +469,15 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
     }
     const size_t unit_bytes = total * stride;
     const size_t owner_bytes = total * sizeof(uint32_t);
-    auto *h_units = static_cast<uint8_t *>(scratch(kHostUnits, unit_bytes + owner_bytes, true));
-    if (!h_units) return MF_ERR_CUDA;
+    // Tables and instance records, units, owners: one buffer, one copy.
+    const size_t meta_used = tables.size() + inst.size() * sizeof(LunnonInstanceDev);
+    const size_t meta_bytes = (meta_used + 255) / 256 * 256;
+    auto *h_all = static_cast<uint8_t *>(
+        scratch(kHostUnits, meta_bytes + unit_bytes + owner_bytes, true));
+    if (!h_all) return MF_ERR_CUDA;
+    std::memcpy(h_all, tables.data(), tables.size());
+    std::memcpy(h_all + tables.size(), inst.data(), meta_used - tables.size());
+    uint8_t *h_units = h_all + meta_bytes;
     auto *h_owner = reinterpret_cast<uint32_t *>(h_units + unit_bytes);
     uint64_t at = 0;
     for (int k = 0; k < num_plans; ++k) {
@@ -441,22 +488,20 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
     const double t1 = now_seconds();
     const BatchKnobs knobs = resolve_knobs(cfg);
     const size_t ws = workspace_bytes(knobs.queue_capacity);
-    const size_t meta_bytes = (tables.size() + inst.size() * sizeof(LunnonInstanceDev) + 255) / 256 * 256;
-    auto *d_units = static_cast<uint8_t *>(scratch(kDevUnits, unit_bytes + owner_bytes, false));
-    auto *d_work = scratch(kDevWork, ws, false);
-    auto *d_meta = static_cast<uint8_t *>(scratch(kDevAux, meta_bytes, false));
-    auto *d_counts = static_cast<uint64_t *>(scratch(kDevCounts, (num_plans + 1) * 8, false));
-    auto *h_counts = static_cast<uint64_t *>(scratch(kHostCounts, (num_plans + 1) * 8 + 64, true));
-    if (!d_units || !d_work || !d_meta || !d_counts || !h_counts) return MF_ERR_CUDA;
+    const size_t out_bytes = counter_bytes(num_plans + 1);
+    auto *d_meta = static_cast<uint8_t *>(
+        scratch(kDevUnits, meta_bytes + unit_bytes + owner_bytes, false));
+    auto *d_counts = static_cast<uint64_t *>(scratch(kDevWork, out_bytes + ws, false));
+    auto *h_counts =
+        static_cast<uint64_t *>(scratch(kHostCounts, out_bytes + sizeof(QueueHeader), true));
+    if (!d_meta || !d_counts || !h_counts) return MF_ERR_CUDA;
+    uint8_t *d_units = d_meta + meta_bytes;
+    void *d_work = reinterpret_cast<uint8_t *>(d_counts) + out_bytes;
     cudaStream_t st = nullptr;
     Timer th, tk, td;
     cudaEventRecord(th.a, st);
-    MF_TRY_CUDA(cudaMemcpyAsync(d_units, h_units, unit_bytes + owner_bytes, cudaMemcpyHostToDevice, st));
-    MF_TRY_CUDA(cudaMemcpyAsync(d_meta, tables.data(), tables.size(), cudaMemcpyHostToDevice, st));
-    auto *d_inst = reinterpret_cast<LunnonInstanceDev *>(d_meta + tables.size());
-    MF_TRY_CUDA(cudaMemcpyAsync(d_inst, inst.data(), inst.size() * sizeof(LunnonInstanceDev),
+    MF_TRY_CUDA(cudaMemcpyAsync(d_meta, h_all, meta_bytes + unit_bytes + owner_bytes,
                                 cudaMemcpyHostToDevice, st));
-    MF_TRY_CUDA(cudaMemsetAsync(d_counts + num_plans, 0, 8, st));
     cudaEventRecord(th.b, st);
     cudaEventRecord(tk.a, st);
     int max_levels = 0, row_levels = 0;
@@ -464,19 +509,18 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
         max_levels = std::max(max_levels, I.n - I.start_leaf);
         if (I.row) row_levels = std::max(row_levels, I.n - I.start_leaf);
     }
-    const uint32_t meta_used = uint32_t(tables.size() + inst.size() * sizeof(LunnonInstanceDev));
-    MF_TRY_CUDA(launch_lunnon_batched(d_meta, meta_used, uint32_t(tables.size()), num_plans,
+    MF_TRY_CUDA(launch_lunnon_batched(d_meta, uint32_t(meta_used), uint32_t(tables.size()), num_plans,
                                       max_levels, row_levels, d_units,
                                       reinterpret_cast<uint32_t *>(d_units + unit_bytes), total,
                                       d_counts, d_counts + num_plans, d_work, knobs, st));
     cudaEventRecord(tk.b, st);
     cudaEventRecord(td.a, st);
-    MF_TRY_CUDA(cudaMemcpyAsync(h_counts, d_counts, (num_plans + 1) * 8, cudaMemcpyDeviceToHost, st));
-    MF_TRY_CUDA(cudaMemcpyAsync(h_counts + num_plans + 1, d_work, sizeof(QueueHeader),
+    MF_TRY_CUDA(cudaMemcpyAsync(h_counts, d_counts, out_bytes + sizeof(QueueHeader),
                                 cudaMemcpyDeviceToHost, st));
     cudaEventRecord(td.b, st);
     MF_TRY_CUDA(cudaStreamSynchronize(st));
-    const QueueHeader *hdr = reinterpret_cast<const QueueHeader *>(h_counts + num_plans + 1);
+    const QueueHeader *hdr = reinterpret_cast<const QueueHeader *>(
+        reinterpret_cast<const uint8_t *>(h_counts) + out_bytes);
     if (int rc = check_queue_header(*hdr, total)) return rc;
     for (int k = 0; k < num_plans; ++k) counts_out[k] = h_counts[k];
     if (stats) {
@@ -557,9 +601,9 @@ struct mf_lunnon_batch {
     uint64_t h2d_bytes = 0;
     uint8_t *d_units = nullptr;
     uint8_t *d_meta = nullptr;
-    uint64_t *d_counts = nullptr;  // num_plans counts + node counter
-    void *d_work = nullptr;
-    uint64_t *h_out = nullptr;     // pinned: counts + node counter + queue header
+    uint64_t *d_counts = nullptr;  // num_plans counts + node counter, then (256-byte aligned)
+    void *d_work = nullptr;        // the workspace
+    uint64_t *h_out = nullptr;     // pinned: what d_counts holds up to the run header
     mf_graph *graph = nullptr;
     cudaStream_t stream = nullptr;
 };
@@ -634,7 +678,6 @@ void mf_lunnon_batch_destroy(mf_lunnon_batch *b) {
     if (b->d_units) cudaFree(b->d_units);
     if (b->d_meta) cudaFree(b->d_meta);
     if (b->d_counts) cudaFree(b->d_counts);
-    if (b->d_work) cudaFree(b->d_work);
     if (b->h_out) cudaFreeHost(b->h_out);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
@@ -702,16 +745,15 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
     MF_TRY_CUDA(cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking));
     MF_TRY_CUDA(cudaMalloc(&b->d_units, std::max<size_t>(host.size(), 16)));
     MF_TRY_CUDA(cudaMalloc(&b->d_meta, (meta.size() + 255) / 256 * 256));
-    MF_TRY_CUDA(cudaMalloc(&b->d_counts, (num_plans + 1) * sizeof(uint64_t)));
-    MF_TRY_CUDA(cudaMalloc(&b->d_work, workspace_bytes(knobs.queue_capacity)));
-    MF_TRY_CUDA(cudaMallocHost(&b->h_out, (num_plans + 1) * sizeof(uint64_t) + sizeof(QueueHeader)));
+    const size_t out_bytes = counter_bytes(num_plans + 1);
+    MF_TRY_CUDA(cudaMalloc(&b->d_counts, out_bytes + workspace_bytes(knobs.queue_capacity)));
+    b->d_work = reinterpret_cast<uint8_t *>(b->d_counts) + out_bytes;
+    MF_TRY_CUDA(cudaMallocHost(&b->h_out, out_bytes + sizeof(QueueHeader)));
     MF_TRY_CUDA(cudaMemcpy(b->d_units, host.data(), host.size(), cudaMemcpyHostToDevice));
     MF_TRY_CUDA(cudaMemcpy(b->d_meta, meta.data(), meta.size(), cudaMemcpyHostToDevice));
     mf_lunnon_batch *raw = b.get();
     rc = capture_graph(
         [&](cudaStream_t s) -> cudaError_t {
-            cudaError_t e = cudaMemsetAsync(raw->d_counts + num_plans, 0, sizeof(uint64_t), s);
-            if (e != cudaSuccess) return e;
             return launch_lunnon_batched(raw->d_meta, uint32_t(meta.size()), inst_offset, num_plans,
                                          max_levels, row_levels, raw->d_units,
                                          reinterpret_cast<uint32_t *>(raw->d_units + unit_bytes),
@@ -737,13 +779,13 @@ int32_t mf_lunnon_batch_run(mf_lunnon_batch *b, uint64_t *counts_out, mf_run_sta
     MF_TRY_CUDA(cudaGraphLaunch(b->graph->exec, b->stream));
     cudaEventRecord(tk.b, b->stream);
     cudaEventRecord(td.a, b->stream);
-    MF_TRY_CUDA(cudaMemcpyAsync(b->h_out, b->d_counts, (np + 1) * sizeof(uint64_t),
-                                cudaMemcpyDeviceToHost, b->stream));
-    MF_TRY_CUDA(cudaMemcpyAsync(b->h_out + np + 1, b->d_work, sizeof(QueueHeader),
+    const size_t out_bytes = counter_bytes(np + 1);
+    MF_TRY_CUDA(cudaMemcpyAsync(b->h_out, b->d_counts, out_bytes + sizeof(QueueHeader),
                                 cudaMemcpyDeviceToHost, b->stream));
     cudaEventRecord(td.b, b->stream);
     MF_TRY_CUDA(cudaStreamSynchronize(b->stream));
-    const QueueHeader *hdr = reinterpret_cast<const QueueHeader *>(b->h_out + np + 1);
+    const QueueHeader *hdr = reinterpret_cast<const QueueHeader *>(
+        reinterpret_cast<const uint8_t *>(b->h_out) + out_bytes);
     if (int rc = check_queue_header(*hdr, b->units)) return rc;
     for (int k = 0; k < np; ++k) counts_out[k] = b->h_out[k];
     if (stats) {
@@ -965,7 +1007,8 @@ int count_cases_host(int n, int start_i, int stop_i, const uint8_t *h_cycles, ui
     Timer th, tk, td;
     cudaEventRecord(th.a, s);
     MF_TRY_CUDA(cudaMemcpyAsync(d_cycles, h_cycles, in_bytes, cudaMemcpyHostToDevice, s));
-    MF_TRY_CUDA(cudaMemsetAsync(d_counts + num, 0, 8, s));
+    const bool clears = mode == 1 && !wide;  // that launch clears the node counter itself
+    if (!clears) MF_TRY_CUDA(cudaMemsetAsync(d_counts + num, 0, 8, s));
     cudaEventRecord(th.b, s);
     cudaEventRecord(tk.a, s);
     if (wide)
@@ -974,7 +1017,7 @@ int count_cases_host(int n, int start_i, int stop_i, const uint8_t *h_cycles, ui
                                     d_work, knobs, s));
     else if (mode == 1)
         MF_TRY_CUDA(launch_sym_batched(edges, n, start_i, stop_i, d_cycles, num, d_counts,
-                                       d_counts + num, d_work, knobs, s));
+                                       d_counts + num, d_work, knobs, s, true));
     else
         MF_TRY_CUDA(launch_sym_plain(edges, start_i, stop_i, d_cycles, num, d_counts, d_counts + num, s));
     cudaEventRecord(tk.b, s);

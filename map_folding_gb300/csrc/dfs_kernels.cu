@@ -121,19 +121,17 @@ __global__ void __launch_bounds__(TPB)
 
 // ------------------------------------------------- persistent kernels ----
 
-__global__ void ring_init_kernel(unsigned long long *seq, unsigned long long capacity) {
-    for (unsigned long long k = blockIdx.x * blockDim.x + threadIdx.x; k < capacity;
-         k += gridDim.x * blockDim.x)
-        seq[k] = k;
+// Ready a launch: the ring's sequence numbers, the run header and `words`
+// counters, in one launch instead of one and two memsets (2-3 us each, a third
+// of a small map's time on the device).
+__global__ void launch_init_kernel(Queue Q, unsigned long long *counts, unsigned long long words) {
+    const unsigned long long step = (unsigned long long)gridDim.x * blockDim.x;
+    const unsigned long long at = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x;
+    for (unsigned long long k = at; k < Q.capacity; k += step) Q.seq[k] = k;
+    for (unsigned long long k = at; k < words; k += step) counts[k] = 0;
+    if (at < 32) reinterpret_cast<unsigned long long *>(Q.hdr)[at] = 0;  // its 256 bytes
 }
 
-// Split items of the persistent kernels start at least this high above the
-// counted level where no row is counted by itself.
-constexpr int kMinRingHeight = 6;
-// Idle lanes of a working warp that go for split items between bookkeepings:
-// every attempt stops the warp for two trips to L2 (500 7x7 cases: 30.8 ms with
-// 1, 29.1 with 16; 6x6: 135 and 131 ms).
-constexpr int kTakeLanes = 16;
 constexpr int kRowLevels = 4;  // Lunnon: levels to go, of a map with rows, from which they pay
 
 // Most cells of a list that the row count takes: all but two of a square's;
@@ -557,7 +555,6 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         const unsigned long long f = warp_sum(finished);
         finished = 0;
         long long queued = 0;
-        int quota = 0;
         if (lane == 0) {
             if (f) atomicAdd(&Q.hdr->completed, f);
             const int idle_now = __popc(idle_mask);
@@ -568,19 +565,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             }
         }
         const HeaderView now(Q.hdr);
-        if (now.init_next() >= num) {
-            queued = (long long)(now.spawn_tail() - now.spawn_head());
-            const long long waiting = now.idle_lanes();
-            const long long want = waiting - queued;
-            if (want > 0) {
-                // This warp's share of what is wanted, twice over: every warp
-                // with work sees the same number, and if all gave all they
-                // could the ring would fill with crumbs.
-                const long long givers = (long long)warps - waiting / 32;
-                const long long q = givers > 0 ? (2 * want + givers - 1) / givers : 32;
-                quota = q < 32 ? int(q) : 32;
-            }
-        }
+        const int quota = split_quota(now, num, warps, queued);
         ring_hint = queued > 0;
         share_miss = false;
         // Feed waiting lanes: busy lanes give away their shallowest untried
@@ -774,10 +759,11 @@ LaunchShape persistent_shape(int sms, int bpsm, int tpb, uint64_t units, int lev
     return LaunchShape{unsigned(blocks), ring < ring_knob ? ring : ring_knob};
 }
 
-cudaError_t reset_queue(const Queue &Q, cudaStream_t stream) {
-    cudaError_t e = cudaMemsetAsync(Q.hdr, 0, 256, stream);
-    if (e != cudaSuccess) return e;
-    ring_init_kernel<<<64, 256, 0, stream>>>(Q.seq, Q.capacity);
+cudaError_t reset_queue(const Queue &Q, uint64_t *counts, uint64_t words, cudaStream_t stream) {
+    const uint64_t most = Q.capacity > words ? Q.capacity : words;
+    const uint64_t blocks = (most + 255) / 256;
+    launch_init_kernel<<<unsigned(blocks < 1024 ? blocks : 1024), 256, 0, stream>>>(
+        Q, reinterpret_cast<unsigned long long *>(counts), words);
     if (g_inject.exchange(0) == MF_FAULT_LOST_SPLIT) phantom_ticket_kernel<<<1, 1, 0, stream>>>(Q.hdr);
     return cudaGetLastError();
 }
@@ -858,10 +844,13 @@ cudaError_t launch_lunnon_plain(const uint8_t *d_table, int n, int dim, int star
 cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int stop_i,
                                const uint8_t *d_cycles, uint64_t num, uint64_t *d_counts,
                                uint64_t *d_nodes, void *d_workspace, const BatchKnobs &knobs,
-                               cudaStream_t stream) {
-    if (num == 0) return reset_queue(carve_queue(d_workspace, knobs.queue_capacity), stream);
-    cudaError_t e = cudaMemsetAsync(d_counts, 0, num * sizeof(uint64_t), stream);
-    if (e != cudaSuccess) return e;
+                               cudaStream_t stream, bool clear_nodes) {
+    // The node counter is cleared with the counts where it follows them (the
+    // host-buffer calls); elsewhere it is the caller's to clear.
+    const bool own_nodes = clear_nodes && d_nodes == d_counts + num;
+    if (num == 0)
+        return reset_queue(carve_queue(d_workspace, knobs.queue_capacity), d_counts, own_nodes, stream);
+    cudaError_t e = cudaSuccess;
     const int sms = device_sm_count();
     // The row count pays while a unit's search still enters the last row from
     // above or near its start; a search to a partial depth has no last row.
@@ -880,7 +869,7 @@ cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int s
         const LaunchShape shape =                                                                \
             persistent_shape(sms, bpsm, TPB, num, stop_i - start_i, knobs.queue_capacity);       \
         const Queue Q = carve_queue(d_workspace, shape.ring);                                    \
-        e = reset_queue(Q, stream);                                                              \
+        e = reset_queue(Q, d_counts, num + own_nodes, stream);                                   \
         if (e != cudaSuccess) return e;                                                          \
         sym_batched_kernel<TPB, LV, TM><<<shape.blocks, TPB, smem, stream>>>(                    \
             d_edges, src, num, counts, nodes, Q, knobs.node_budget, knobs.wait_limit);          \
@@ -917,9 +906,11 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
                                   const uint8_t *d_states, const uint32_t *d_state_owner,
                                   uint64_t num, uint64_t *d_counts, uint64_t *d_nodes,
                                   void *d_workspace, const BatchKnobs &knobs, cudaStream_t stream) {
-    cudaError_t e = cudaMemsetAsync(d_counts, 0, size_t(num_inst) * sizeof(uint64_t), stream);
-    if (e != cudaSuccess) return e;
-    if (num == 0) return reset_queue(carve_queue(d_workspace, knobs.queue_capacity), stream);
+    // The node counter follows the counts and is cleared with them.
+    const uint64_t words = uint64_t(num_inst) + (d_nodes == d_counts + num_inst ? 1 : 0);
+    if (num == 0)
+        return reset_queue(carve_queue(d_workspace, knobs.queue_capacity), d_counts, words, stream);
+    cudaError_t e = cudaSuccess;
     const int sms = device_sm_count();
     const uint32_t mb = (meta_bytes + 15) / 16 * 16;
     const LunnonSource src{d_states, d_state_owner, nullptr, lunnon_state_stride(64)};
@@ -935,7 +926,7 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
         const LaunchShape shape =                                                                \
             persistent_shape(sms, bpsm, TPB, num, max_levels, knobs.queue_capacity);             \
         const Queue Q = carve_queue(d_workspace, shape.ring);                                    \
-        e = reset_queue(Q, stream);                                                              \
+        e = reset_queue(Q, d_counts, words, stream);                                             \
         if (e != cudaSuccess) return e;                                                          \
         lunnon_batched_kernel<TPB, LV, TM><<<shape.blocks, TPB, smem, stream>>>(                 \
             d_meta, mb, inst_offset, src, num, counts, nodes, Q, knobs.node_budget,             \

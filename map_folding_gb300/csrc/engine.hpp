@@ -235,7 +235,7 @@ cudaError_t launch_sym_wide(const uint8_t *d_wide_edges, int start_i, int stop_i
 cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int stop_i,
                                const uint8_t *d_cycles, uint64_t num, uint64_t *d_counts,
                                uint64_t *d_nodes, void *d_workspace, const BatchKnobs &knobs,
-                               cudaStream_t stream);
+                               cudaStream_t stream, bool clear_nodes = false);
 cudaError_t launch_lunnon_plain(const uint8_t *d_table, int n, int dim, int start_leaf,
                                 const uint8_t *d_states, uint32_t stride, uint64_t num,
                                 uint64_t *d_per_state, uint64_t *d_total, uint64_t *d_nodes,

@@ -305,7 +305,10 @@ __global__ void __launch_bounds__(TPB)
     const unsigned lt_mask = (1u << lane) - 1u;
     constexpr int kOwner = kWideWords, kMaskW = kWideWords + 1, kRoot = kWideWords + 5,
                   kRowOk = kWideWords + 6;
-    bool busy = false, fresh = false, init_left = true;
+    // With fewer units than lanes every warp takes its share of them.
+    const unsigned long long warps = (unsigned long long)gridDim.x * (TPB / 32);
+    bool busy = false, fresh = false;
+    bool init_left = (unsigned long long)lane * warps < num;
     int lvl = start_i, root = start_i, eval = start_i;
     uint32_t owner = 0;
     unsigned long long leaves = 0, nodes = 0, finished = 0, started = 0;
@@ -354,17 +357,17 @@ __global__ void __launch_bounds__(TPB)
         return S.get(s);
     };
 
-    auto donate = [&]() {
+    auto donate = [&](int quota) {
         int s = root;
         const Mask128 m = shallowest(s);
         const bool can = !w_zero(m) && (row_level != kNoRow ? row_level - s >= kRowSplit
-                                                            : last - s >= kMinSplitHeight);
-        const unsigned donors = __ballot_sync(kFull, can);
+                                                            : last - s >= kMinRingHeight);
+        const unsigned donors = shallowest_lanes(can, s, quota);
         if (!donors) return;
         unsigned long long first = 0;
         const int got = ring_claim(Q, &Q.hdr->spawn_tail, __popc(donors), false, first);
         const int rank = __popc(donors & lt_mask);
-        if (!can || rank >= got) return;
+        if (!((donors >> lane) & 1u) || rank >= got) return;
         for (int l = lvl; l >= s; --l) L.put(S.pick(l), L.get(l));
         uint32_t w[kWideRecordWords];
 #pragma unroll
@@ -487,7 +490,8 @@ __global__ void __launch_bounds__(TPB)
         if (__popc(unfed) >= kShareLanes && unfed != kFull && !share_miss) share_miss = !share(unfed);
         if (ring_hint) {
             const unsigned need = __ballot_sync(kFull, !busy && !init_left);
-            if (need && take_splits(need)) ring_hint = false;
+            if (need && (__popc(need) >= kTakeLanes || round + 1 >= period) && take_splits(need))
+                ring_hint = false;
         }
         const bool bookkeeping = ++round >= period;
         if (!__any_sync(kFull, busy)) {
@@ -502,20 +506,15 @@ __global__ void __launch_bounds__(TPB)
                 }
             }
             const unsigned need = __ballot_sync(kFull, !init_left);
-            if (need) take_splits(need);
+            const HeaderView now(Q.hdr);
+            if (need && now.spawn_tail() != now.spawn_head()) take_splits(need);
             if (__any_sync(kFull, busy) || __any_sync(kFull, init_left)) {
                 idle_rounds = 0;
                 nap = 256;
                 continue;
             }
-            int stop = 0;
-            if (lane == 0) {
-                const unsigned long long total = num + vload(&Q.hdr->spawn_tail);
-                stop = (vload(&Q.hdr->init_next) >= num && vload(&Q.hdr->completed) >= total) ||
-                       *reinterpret_cast<volatile unsigned int *>(&Q.hdr->error) != 0u ||
-                       ++idle_rounds > wait_limit;
-            }
-            stop = __shfl_sync(kFull, stop, 0);
+            const bool stop = (now.init_next() >= num && now.completed() >= num + now.spawn_tail()) ||
+                              now.error() != 0u || ++idle_rounds > wait_limit;
             if (stop) break;
             __nanosleep(nap);
             if (nap < 8192) nap <<= 1;
@@ -569,7 +568,6 @@ __global__ void __launch_bounds__(TPB)
         const unsigned idle_mask = __ballot_sync(kFull, !busy);
         const unsigned long long f = warp_sum(finished);
         finished = 0;
-        long long want = 0, queued = 0;
         if (lane == 0) {
             if (f) atomicAdd(&Q.hdr->completed, f);
             const int idle_now = __popc(idle_mask);
@@ -578,15 +576,13 @@ __global__ void __launch_bounds__(TPB)
                           (unsigned long long)(long long)(idle_now - reported_idle));
                 reported_idle = idle_now;
             }
-            if (vload(&Q.hdr->init_next) >= num) {
-                queued = (long long)(vload(&Q.hdr->spawn_tail) - vload(&Q.hdr->spawn_head));
-                want = *reinterpret_cast<volatile long long *>(&Q.hdr->idle_lanes) - queued;
-            }
         }
-        want = __shfl_sync(kFull, want, 0);
-        ring_hint = __shfl_sync(kFull, queued, 0) > 0;
+        const HeaderView now(Q.hdr);
+        long long queued = 0;
+        const int quota = split_quota(now, num, warps, queued);
+        ring_hint = queued > 0;
         share_miss = false;
-        if (want > 0) donate();
+        if (quota > 0) donate(quota);
     }
 
     if (lane == 0 && reported_idle)
