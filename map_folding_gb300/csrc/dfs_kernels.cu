@@ -516,7 +516,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             const unsigned at = __ballot_sync(kFull, here);
             if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
                 const int K0 = last - eval;
-                uint32_t C = 0, R = 0, H = 0, counted = 0;
+                uint32_t C = 0, counted = 0;
+                typename RowTail::Hist R = 0, H = 0;
                 uint32_t W[RowTail::kRow] = {};
                 bool ok = false;
                 tail.prepare_setup();

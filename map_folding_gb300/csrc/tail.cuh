@@ -50,9 +50,12 @@ namespace {
 // BITS: of a face number, enough for half as many faces as cells.
 template <int TMAX, int CELLS, int FILL, int BITS>
 struct TailLayout {
-    static_assert(CELLS <= (BITS == 5 ? 63 : 80) && FILL <= 32 && TMAX >= 2 && TMAX <= 8, "tail layout");
+    static_assert(CELLS <= (BITS == 5 ? 63 : 80) && FILL <= 32 && TMAX >= 2 && TMAX <= 9, "tail layout");
     static constexpr int kCap = FILL + 32;
-    __host__ __device__ static constexpr int quads(int k) { return (3 + k + 3) / 4; }
+    // Words of a frame ahead of its W: C, R, H and, where these pass 32 bits,
+    // their high bits.
+    static constexpr int kHead = TMAX > 8 ? 4 : 3;
+    __host__ __device__ static constexpr int quads(int k) { return (kHead + k + 3) / 4; }
     __host__ __device__ static constexpr int cap(int k) { return k == TMAX - 1 ? 32 : kCap; }
     __host__ __device__ static constexpr int frames(int k) {  // offset of level k's queue
         int at = kFrames;
@@ -93,10 +96,23 @@ struct TailPages {
 // kSym: a square's side, always of TMAX cells; else rows of a Lunnon map, of up
 // to TMAX leaves (a longer row starts inside), whose gap on the sentinel counts
 // as a node and is not searched.
+template <bool kLong>
+struct HistWord {
+    using type = uint32_t;
+};
+template <>
+struct HistWord<true> {
+    using type = uint64_t;
+};
+
 template <bool kSym, int TMAX, int CELLS, int FILL, int BITS = 5>
 struct Tail {
     using Y = TailLayout<TMAX, CELLS, FILL, BITS>;
     static constexpr int kRow = TMAX;
+    // R: the gap numbers of the earlier picks, five bits each, the latest
+    // lowest; H: the h bits, and the root's slot above them.
+    using Hist = typename HistWord<(TMAX > 8)>::type;
+    static constexpr int kSlotShift = TMAX > 8 ? 56 : 27;  // the top of the last frame word
     uint8_t *area;
     int lane;
     int cnt[TMAX];  // frames queued per level 1 .. TMAX-1 (warp-uniform)
@@ -131,7 +147,7 @@ struct Tail {
     template <class List, class WOf>
     __device__ __forceinline__ bool setup(const List &L, int placed, int K0, const TailPages &pg,
                                           WOf &&w, int prev, uint32_t &C, uint32_t (&W)[TMAX],
-                                          uint32_t &R, uint32_t &H) const {
+                                          Hist &R, Hist &H) const {
         constexpr uint32_t kField = (1u << BITS) - 1;
         constexpr uint32_t kIds = (1u << (3 * BITS)) - 1;
         uint32_t *pre = word(Y::kPre) + lane;
@@ -223,7 +239,7 @@ struct Tail {
         }
         if (!kSym) word(Y::kTop)[lane] = first_in | uint32_t(prev >= 0 ? TMAX : K0) << 8;
         R = 0;
-        H = uint32_t(lane) << 27;
+        H = Hist(lane) << kSlotShift;
         if (prev >= 0) {
             // v_{t-1} is a cell of the list: its face on the page of the next
             // arc, and it stands in for all earlier picks (an arc between two
@@ -237,10 +253,10 @@ struct Tail {
                 m &= (fp >> j) & 1 ? plane : ~plane;
             }
             C &= m;
-            const uint32_t before = pre[prev * 32] >> 24;
+            const Hist before = pre[prev * 32] >> 24;
 #pragma unroll
-            for (int j = 0; j < 6; ++j) R |= before << (5 * j);
-            H |= (~0u << hbit(0, K0 + 1)) & 0x07ffffffu;
+            for (int j = 0; j < (TMAX > 8 ? 7 : 6); ++j) R |= before << (5 * j);
+            H |= (~Hist(0) << hbit(0, K0 + 1)) & ((Hist(1) << hbit(0, TMAX)) - 1);
         }
         return true;
     }
@@ -248,7 +264,7 @@ struct Tail {
     // Put the root frames of the lanes in `have` into their levels' queues
     // (all lanes call; the set-up's scratch is given up here).
     __device__ __forceinline__ void enqueue_roots(bool have, int K0, uint32_t C, uint32_t (&W)[TMAX],
-                                                  uint32_t R, uint32_t H) {
+                                                  Hist R, Hist H) {
         word(Y::kAcc)[lane] = 0;
         __syncwarp();
         push_roots<TMAX - 1>(have, K0, C, W, R, H);
@@ -257,7 +273,7 @@ struct Tail {
 
     template <int K>
     __device__ __forceinline__ void push_roots(bool have, int K0, uint32_t C, uint32_t (&W)[TMAX],
-                                               uint32_t R, uint32_t H) {
+                                               Hist R, Hist H) {
         if constexpr (K >= 1) {
             cnt[K] = 0;
             push<K>(have && K0 == K && C != 0, C, W, R, H);
@@ -266,8 +282,8 @@ struct Tail {
     }
 
     template <int K>
-    __device__ __forceinline__ void push(bool mine, uint32_t C, const uint32_t (&W)[TMAX], uint32_t R,
-                                         uint32_t H) {
+    __device__ __forceinline__ void push(bool mine, uint32_t C, const uint32_t (&W)[TMAX], Hist R,
+                                         Hist H) {
         const unsigned m = __ballot_sync(kFull, mine);
         if (!m) return;
         const int at = cnt[K] + __popc(m & ((1u << lane) - 1));
@@ -275,10 +291,12 @@ struct Tail {
         if (mine) {
             uint32_t w[4 * Y::quads(K)] = {};
             w[0] = C;
-            w[1] = R;
-            w[2] = H;
+            w[1] = uint32_t(R);
+            w[2] = uint32_t(H);
+            if constexpr (TMAX > 8)
+                w[3] = uint32_t(R >> 32) | uint32_t(H >> 32) << 3;  // 3 bits, 3 bits and the slot
 #pragma unroll
-            for (int e = 0; e < K; ++e) w[3 + e] = W[e];
+            for (int e = 0; e < K; ++e) w[Y::kHead + e] = W[e];
             uint4 *q = reinterpret_cast<uint4 *>(area + Y::frames(K)) + at;
 #pragma unroll
             for (int j = 0; j < Y::quads(K); ++j)
@@ -289,7 +307,7 @@ struct Tail {
     // Idle lanes (C == 0) take frames of level K.
     template <int K>
     __device__ __forceinline__ void refill(uint32_t &C, uint32_t (&W)[TMAX], uint32_t (&b)[TMAX],
-                                           uint32_t &R, uint32_t &H) {
+                                           Hist &R, Hist &H) {
         const unsigned idle = __ballot_sync(kFull, C == 0);
         const int want = __popc(idle);
         const int take = want < cnt[K] ? want : cnt[K];
@@ -309,16 +327,21 @@ struct Tail {
             C = w[0];
             R = w[1];
             H = w[2];
+            if constexpr (TMAX > 8) {
+                R |= Hist(w[3] & 7) << 32;
+                H |= Hist(w[3] >> 3) << 32;
+            }
 #pragma unroll
-            for (int e = 0; e < K; ++e) W[e] = w[3 + e];
+            for (int e = 0; e < K; ++e) W[e] = w[Y::kHead + e];
 #pragma unroll
-            for (int e = K + 1; e < TMAX; ++e) b[e] = 1u << ((R >> (5 * (e - K - 1))) & 31);
+            for (int e = K + 1; e < TMAX; ++e)
+                b[e] = 1u << (uint32_t(R >> (5 * (e - K - 1))) & 31);
         }
         __syncwarp();
     }
 
     // A(es, ex): the gaps whose piece seen by level ex is after v_es.
-    __device__ static __forceinline__ uint32_t after(const uint32_t (&b)[TMAX], uint32_t H, int ex,
+    __device__ static __forceinline__ uint32_t after(const uint32_t (&b)[TMAX], Hist H, int ex,
                                                      int es) {
         const uint32_t n = 0u - b[es];
         return (H >> hbit(ex, es)) & 1 ? n : n + n;
@@ -331,7 +354,7 @@ struct Tail {
     // placed cells' frames go on to the next level.
     template <int K>
     __device__ __forceinline__ void levels(int start, uint32_t &C, uint32_t (&W)[TMAX],
-                                           uint32_t (&b)[TMAX], uint32_t &R, uint32_t &H,
+                                           uint32_t (&b)[TMAX], Hist &R, Hist &H,
                                            uint32_t &nodes) {
         if constexpr (K >= 1) {
             if (K <= start) {
@@ -347,7 +370,7 @@ struct Tail {
                 }
                 uint32_t next = 0;
                 if (bt) {
-                    const int slot = int(H >> 27);
+                    const int slot = int(H >> kSlotShift);
                     const uint32_t info = kSym ? 0 : word(Y::kTop)[slot];
                     const int r = 31 - __clz(int(bt));
                     const uint32_t *before = word(Y::kBefore) + slot;
@@ -368,7 +391,7 @@ struct Tail {
                         const bool in = (pe >= bt) != (pe > pt);
                         W[e] &= in ? inside : outside;
                         if constexpr (K >= 2)
-                            if (in != up) H |= 1u << hbit(e, K);
+                            if (in != up) H |= Hist(1) << hbit(e, K);
                     }
                     next = face & W[K - 1];
 #pragma unroll
@@ -388,7 +411,8 @@ struct Tail {
                         next = 0;
                     }
                     b[K] = bt;
-                    R = (R << 5) | uint32_t(r);
+                    R = (R << 5) | Hist(r);
+                    if constexpr (TMAX > 8) R &= (Hist(1) << 35) - 1;
                 }
                 C = next;
             }
@@ -407,7 +431,8 @@ struct Tail {
             for (int k = TMAX - 1; k >= 1; --k)
                 if (cnt[k] >= FILL) start = k;  // ... or the deepest full one
             if (start == 0) return;
-            uint32_t C = 0, R = 0, H = 0;
+            uint32_t C = 0;
+            Hist R = 0, H = 0;
             uint32_t W[TMAX] = {}, b[TMAX] = {};
             levels<TMAX - 1>(start, C, W, b, R, H, nodes);
         }

@@ -160,11 +160,13 @@ struct LocalStackW {
     __device__ __forceinline__ void set_pick(int lvl, int j) { chosen[lvl - base] = uint8_t(j); }
 };
 
-// Row counting on the 9x9 board: its last eight cells (the layout's most; a
-// row of nine starts with the list walk).
-constexpr int kWideRow = 8;
+// Row counting on the 9x9 board.  A level is full at eight frames: three CTAs
+// fit on an SM then, two with the 64-bit kernels' sixteen.  (Counting only the
+// last eight cells, whose roots are a fifth the size: 582 ms for 2,000 cases at
+// 48 cells, and 636 ms by list alone.)
+constexpr int kWideRow = 9;
 constexpr int kWideTailCells = 79;
-using WideTail = Tail<true, kWideRow, kWideTailCells, kTailFill, 6>;
+using WideTail = Tail<true, kWideRow, kWideTailCells, 8, 6>;
 
 template <int TPB, int LEVELS, bool kRow>
 struct WideStack {
@@ -273,7 +275,7 @@ __device__ __forceinline__ void wide_put(uint4 *slots, const Queue &Q, unsigned 
 // Split record: list words 0..kWideWords-1, owner, untried mask (4 words),
 // level, whether the row may be counted on masks.
 // idle lanes, and the same leaving rule; lanes of a warp share as there.  With
-// kRow the last cells of the 9x9 row are counted on masks (tail.cuh).
+// kRow the 9x9 board's last row is counted on masks (tail.cuh).
 template <int TPB, int LEVELS, bool kRow>
 __global__ void __launch_bounds__(TPB)
     sym_wide_kernel(const uint8_t *__restrict__ edges, int start_i, int last,
@@ -538,12 +540,14 @@ __global__ void __launch_bounds__(TPB)
             const unsigned at = __ballot_sync(kFull, here);
             if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
                 uint32_t W[WideTail::kRow] = {};
-                uint32_t c = 0, r = 0, h = 0, counted = 0;
+                uint32_t c = 0, counted = 0;
+                WideTail::Hist r = 0, h = 0;
                 bool ok = false;
                 tail.prepare_setup();
                 if (here) {
                     auto w = [&](int e) -> int { return pages.b[last - e]; };
-                    ok = tail.setup(L, eval, last - eval, pages, w, eval - 1, c, W, r, h);
+                    ok = tail.setup(L, eval, last - eval, pages, w, eval > row_first ? eval - 1 : -1, c, W,
+                                    r, h);
                     if (ok) counted = __popc(c) + 1;
                     else by_walk = true;
                 }
