@@ -141,9 +141,14 @@ __host__ __device__ constexpr int tail_cells() {
     return kSym && TMAX > 2 ? TMAX * TMAX - 2 : kRowLeaves - 1;
 }
 
+template <bool kSym>
+__host__ __device__ constexpr int tail_fill() {
+    return kSym ? kTailFill : kLunnonTailFill;
+}
+
 template <bool kSym, int TMAX>
 __host__ __device__ constexpr size_t tail_bytes(int tpb) {
-    if constexpr (TMAX > 0) return size_t(tpb / 32) * TailLayout<TMAX, tail_cells<kSym, TMAX>(), kTailFill, 5>::kBytes;
+    if constexpr (TMAX > 0) return size_t(tpb / 32) * TailLayout<TMAX, tail_cells<kSym, TMAX>(), tail_fill<kSym>(), 5>::kBytes;
     else return 0;
 }
 
@@ -212,7 +217,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                              reinterpret_cast<const uint32_t *>(s_tables + 4 * kSymCells),
                              s_tables + 8 * kSymCells, sym.start_i};
     LunnonRules lrules{s_tables, 0, 0};
-    using RowTail = Tail<kSym, (TMAX > 0 ? TMAX : 2), tail_cells<kSym, TMAX>(), kTailFill>;
+    using RowTail =
+        Tail<kSym, (TMAX > 0 ? TMAX : 2), tail_cells<kSym, TMAX>(), tail_fill<kSym>()>;
     RowTail tail;
     tail.area = tail_area;
     tail.lane = lane;
@@ -588,7 +594,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
 }
 
 template <int TPB, int LEVELS, int TMAX>
-__global__ void __launch_bounds__(TPB)
+__global__ void __launch_bounds__(TPB, TMAX > 0 ? 4 : 1)
     sym_batched_kernel(const uint8_t *__restrict__ edges, SymSource src, unsigned long long num,
                        unsigned long long *counts, unsigned long long *nodes_out, Queue Q,
                        uint32_t period, uint32_t wait_limit) {

@@ -26,6 +26,7 @@
 
 #include "dfs_core.cuh"
 #include "engine.hpp"
+#include "tail.cuh"
 
 namespace mf {
 namespace {
@@ -46,7 +47,8 @@ struct alignas(16) SlotInfo {  // 32 bytes
     int32_t base;              // first level of the request's units
     int32_t last;              // level counted by popcount
     uint32_t table_off;        // Lunnon: neighbour table in the table arena
-    uint32_t weight;           // leaves per counted position (Lunnon: n)
+    uint16_t weight;           // leaves per counted position (Lunnon: n)
+    uint16_t row;              // cells of the last row, counted by itself (0: none)
     uint32_t seq;              // request sequence number
 };
 
@@ -100,18 +102,33 @@ struct ServeArgs {
     uint32_t wait_limit;
 };
 
-template <int TPB, int LEVELS>
+// Squares of 6 to 8 and Lunnon rows of up to 8 leaves share the rows' queues;
+// a request's nodes are its own, so they are added up per root.
+constexpr int kServeRow = 8;
+using ServeTail = Tail<false, kServeRow, kServeRow * kServeRow - 2, kTailFill, 5, true>;
+
+// The last row of a request is counted on masks (tail.cuh) and the lanes of a
+// warp share their work, as in the batched kernels; the mask stack is in local
+// memory, which leaves the shared memory to the rows.
+template <int TPB>
 __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
     extern __shared__ __align__(16) uint8_t smem[];
     constexpr size_t kTables = 3 * kSymTables;  // n = 6, 7, 8
     for (int b = 0; b < 3; ++b) stage_sym_tables<TPB>(smem + b * kSymTables, A.edges + b * 4 * kSymCells);
     __syncthreads();
-    using C = Carve<TPB, 17, LEVELS>;
+    using C = Carve<TPB, 17, 0>;
     const List<TPB> L = C::list(smem, kTables);
-    SmemStack<TPB, LEVELS> S = C::stack(smem, kTables);
+    LocalStack S;
+    S.base = 0;
 
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
+    ServeTail tail;
+    tail.area = smem + kTables + C::kThreadBytes + threadIdx.x / 32 * ServeTail::Y::kBytes;
+    tail.lane = lane;
+    TailPages pages{};
+    int row = 0, row_level = kNoRow;
+    bool by_walk = false, share_miss = false;
     bool busy = false, fresh = false;
     int lvl = 0, root = 0, last = 0, eval = 0;
     uint32_t slot = 0, kind = 0, weight = 1, my_seq = 0;
@@ -142,8 +159,20 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
         my_seq = I.seq;
         last = I.last;
         S.base = I.base;
-        if (kind == 0) srules = sym_rules(smem + (I.n - 6) * kSymTables);
-        else lrules = LunnonRules{A.tables + I.table_off, I.n, I.dim};
+        row = I.row;
+        row_level = row > 0 ? last + 1 - (row < kServeRow ? row : kServeRow) : kNoRow;
+        by_walk = false;
+        if (kind == 0) {
+            const uint8_t *edge = smem + (I.n - 6) * kSymTables;
+            srules = sym_rules(edge);
+            if (row > 0) pages = sym_row_pages(edge, last, kSymCells);
+        } else {
+            lrules = LunnonRules{A.tables + I.table_off, I.n, I.dim};
+            const int w = I.n + 1;
+            pages.a1 = lrules.table + I.n * w;
+            pages.a0 = lrules.table + (I.n - 1) * w;
+            pages.b = lrules.table + (w + I.n) * w;
+        }
     };
 
     // Count a finished unit or split item into its request; the lane that
@@ -168,6 +197,36 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
 
     auto evaluate = [&]() -> uint64_t {
         return kind == 0 ? srules.gaps(L, eval, nodes) : lrules.gaps(L, eval, nodes);
+    };
+
+    // share_in_warp; a piece counts as a work item of its request (the giver
+    // adds it, ahead of what it will itself take off).
+    auto share = [&](unsigned idle) -> bool {
+        uint32_t its_slot = 0;
+        uint64_t its_mult = 0;
+        unsigned givers = 0;
+        return share_in_warp(
+            L, S, busy && !fresh, root, lvl,
+            row_level != kNoRow ? row_level - kRowShare : last - kMinShareHeight, idle,
+            [&](int from, bool take) {
+                its_slot = __shfl_sync(kFull, slot, from);
+                its_mult = __shfl_sync(kFull, mult, from);
+                givers = __reduce_or_sync(kFull, take ? 1u << from : 0u);
+                if ((givers >> lane) & 1u) {
+                    atomicAdd(reinterpret_cast<unsigned long long *>(A.pending + slot), 1ULL);
+                    __threadfence();  // before any lane takes the piece off again
+                }
+            },
+            [&](int level, uint64_t mask) {
+                set_slot(its_slot);
+                mult = its_mult;
+                root = level;
+                unit_nodes0 = nodes;
+                S.set(root, mask);
+                eval = advance(L, S, lvl, root);
+                fresh = false;
+                busy = true;
+            });
     };
 
     for (;;) {
@@ -256,6 +315,8 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
             }
             if (g2 < __popc(rest)) ring_hint = false;
         }
+        const unsigned unfed = __ballot_sync(kFull, !busy);
+        if (__popc(unfed) >= kShareLanes && unfed != kFull && !share_miss) share_miss = !share(unfed);
         const bool bookkeeping = ++round >= A.period;
         if (!__any_sync(kFull, busy)) {
             int stop = 0;
@@ -290,8 +351,10 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
         }
         nap = 256;
         stuck_rounds = 0;
-        if (busy) {
+        auto at_row = [&]() { return busy && eval >= row_level && eval < last && !by_walk; };
+        if (busy && !at_row()) {
             const uint64_t g = evaluate();
+            by_walk = false;
             eval = apply_advance(L, S, lvl, eval, root, last, fresh, g, leaves);
             fresh = false;
             if (eval < 0) {
@@ -299,8 +362,46 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
                 busy = false;
             }
         }
+        const bool here = at_row();
+        const unsigned at = __ballot_sync(kFull, here);
+        if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
+            uint32_t W[ServeTail::kRow] = {};
+            uint32_t c = 0, counted = 0, none = 0;
+            ServeTail::Hist r = 0, h = 0;
+            bool ok = false;
+            tail.prepare_setup();
+            if (here) {
+                auto w = [&](int e) -> int {
+                    return kind == 0 ? int(pages.b[last - e]) : last - e - row;
+                };
+                const int prev = eval > last + 1 - row ? eval - 1 : -1;
+                ok = tail.setup(L, eval, last - eval, pages, w, prev, c, W, r, h, kind != 0);
+                if (ok) {
+                    counted = __popc(c) + (kind == 0 ? 1 : 0);
+                    if (kind != 0) c &= ~(tail.word(ServeTail::Y::kTop)[lane] & 1);
+                } else {
+                    by_walk = true;
+                }
+            }
+            tail.enqueue_roots(ok, last - eval, c, W, r, h);
+            tail.drain(none);
+            __syncwarp();
+            if (ok) {
+                nodes += counted + tail.word(ServeTail::Y::kRootNodes)[lane];
+                leaves += tail.word(ServeTail::Y::kAcc)[lane];
+                eval = apply_advance(L, S, lvl, eval, root, last, fresh, 0, leaves);
+                fresh = false;
+                if (eval < 0) {
+                    finish();
+                    busy = false;
+                }
+            }
+            __syncwarp();
+            round += kTailRounds;
+        }
         if (!bookkeeping) continue;
         round = 0;
+        share_miss = false;
         const unsigned idle_mask = __ballot_sync(kFull, !busy);
         long long want = 0, queued = 0;
         unsigned oldest = 0;
@@ -327,7 +428,9 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
             // to keep its stock of split items.
             int s = root;
             const uint64_t m = busy && !fresh ? shallowest_siblings(S, root, lvl, s) : 0;
-            const bool can = busy && !fresh && m != 0 && last - s >= kMinSplitHeight &&
+            const bool can = busy && !fresh && m != 0 &&
+                             (row_level != kNoRow ? row_level - s >= kRowSplit
+                                                  : last - s >= kMinRingHeight) &&
                              (want > 0 || my_seq == oldest);
             const unsigned donors = __ballot_sync(kFull, can);
             if (donors) {
@@ -495,7 +598,7 @@ cudaError_t launch_server_kernel(mf_server *s) {
     A.Q = s->Q;
     A.period = s->cfg.node_budget;
     A.wait_limit = 1u << 20;
-    serve_kernel<kServeTPB, kServeLevels>
+    serve_kernel<kServeTPB>
         <<<unsigned(s->sms * s->blocks_per_sm), kServeTPB, s->smem, s->kstream>>>(A);
     return cudaGetLastError();
 }
@@ -746,13 +849,14 @@ int make_server(const mf_server_config *cfg, mf_server **out) {
     MF_TRY_CUDA(cudaMallocHost(&s->h_stage, s->stage_cap * sizeof(ServeUnit)));
     std::memset(static_cast<void *>(s->h_done), 0, c.max_requests * sizeof(DoneRec));
     MF_TRY_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void **>(&s->d_done), s->h_done, 0));
-    s->smem = 3 * kSymTables + Carve<kServeTPB, 17, kServeLevels>::kThreadBytes;
+    s->smem = 3 * kSymTables + Carve<kServeTPB, 17, 0>::kThreadBytes +
+              kServeTPB / 32 * ServeTail::Y::kBytes;
     int optin = 0;
     MF_TRY_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, s->device));
-    MF_TRY_CUDA(cudaFuncSetAttribute(serve_kernel<kServeTPB, kServeLevels>,
+    MF_TRY_CUDA(cudaFuncSetAttribute(serve_kernel<kServeTPB>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
     MF_TRY_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-        &s->blocks_per_sm, serve_kernel<kServeTPB, kServeLevels>, kServeTPB, s->smem));
+        &s->blocks_per_sm, serve_kernel<kServeTPB>, kServeTPB, s->smem));
     if (s->blocks_per_sm < 1) {
         set_error("the server kernel does not fit on an SM");
         return MF_ERR_CUDA;
@@ -876,6 +980,7 @@ int32_t mf_server_submit_sym(mf_server *s, int32_t n, int32_t expanded_n, uint64
     r->info.base = plan->start_i;
     r->info.last = n * n - 1;
     r->info.weight = 1;
+    r->info.row = uint16_t(n);
     r->factor = (unsigned __int128)(n * n);
     return submit(s, r, request_id);
 }
@@ -920,7 +1025,8 @@ int32_t mf_server_submit_lunnon(mf_server *s, const int32_t *dims, int32_t ndim,
     r->info.dim = t.dim;
     r->info.base = depth + 1;
     r->info.last = t.n;
-    r->info.weight = uint32_t(t.n);
+    r->info.weight = uint16_t(t.n);
+    r->info.row = t.dim == 2 && t.p[0] >= 3 && t.p[1] >= 2 && t.n <= kRowLeaves ? uint16_t(t.p[0]) : 0;
     r->factor = 1;
     return submit(s, r, request_id);
 }

@@ -65,9 +65,11 @@ struct TailLayout {
     static constexpr int kPlane = 0;                         // 2 pages x BITS planes
     static constexpr int kBefore = kPlane + 2 * BITS * 128;  // P of each level
     static constexpr int kTop = kBefore + TMAX * 128;        // Lunnon: bit 0 the gap on the sentinel,
+                                                             // bit 1 leaves are nodes too,
                                                              // << 8 the first level with an arc
     static constexpr int kAcc = kTop + 128;                  // leaves of each root
-    static constexpr int kFrames = kAcc + 128;
+    static constexpr int kRootNodes = kAcc + 128;            // nodes of each root (if asked for)
+    static constexpr int kFrames = kRootNodes + 128;
     // Scratch of the set-up, in the frames' place (they are empty then): a word
     // per cell (the face numbers before it, later also the gaps of U before it)
     // and 16 words of face numbers per gap of U.
@@ -95,7 +97,8 @@ struct TailPages {
 
 // kSym: a square's side, always of TMAX cells; else rows of a Lunnon map, of up
 // to TMAX leaves (a longer row starts inside), whose gap on the sentinel counts
-// as a node and is not searched.
+// as a node and is not searched; or, where squares' sides shorter than TMAX are
+// among them, both (the request server).
 template <bool kLong>
 struct HistWord {
     using type = uint32_t;
@@ -105,7 +108,8 @@ struct HistWord<true> {
     using type = uint64_t;
 };
 
-template <bool kSym, int TMAX, int CELLS, int FILL, int BITS = 5>
+// With kRootNodes the nodes too are added up per root, not per lane.
+template <bool kSym, int TMAX, int CELLS, int FILL, int BITS = 5, bool kRootNodes = false>
 struct Tail {
     using Y = TailLayout<TMAX, CELLS, FILL, BITS>;
     static constexpr int kRow = TMAX;
@@ -147,7 +151,7 @@ struct Tail {
     template <class List, class WOf>
     __device__ __forceinline__ bool setup(const List &L, int placed, int K0, const TailPages &pg,
                                           WOf &&w, int prev, uint32_t &C, uint32_t (&W)[TMAX],
-                                          Hist &R, Hist &H) const {
+                                          Hist &R, Hist &H, bool lunnon = !kSym) const {
         constexpr uint32_t kField = (1u << BITS) - 1;
         constexpr uint32_t kIds = (1u << (3 * BITS)) - 1;
         uint32_t *pre = word(Y::kPre) + lane;
@@ -237,7 +241,8 @@ struct Tail {
             if (e == K0) C = m;
             word(Y::kBefore)[e * 32 + lane] = e <= K0 ? (1u << (pre[w(e) * 32] >> 24)) - 1 : 0;
         }
-        if (!kSym) word(Y::kTop)[lane] = first_in | uint32_t(prev >= 0 ? TMAX : K0) << 8;
+        if (!kSym)
+            word(Y::kTop)[lane] = (lunnon ? first_in | 2u : 0u) | uint32_t(prev >= 0 ? TMAX : K0) << 8;
         R = 0;
         H = Hist(lane) << kSlotShift;
         if (prev >= 0) {
@@ -266,6 +271,7 @@ struct Tail {
     __device__ __forceinline__ void enqueue_roots(bool have, int K0, uint32_t C, uint32_t (&W)[TMAX],
                                                   Hist R, Hist H) {
         word(Y::kAcc)[lane] = 0;
+        if (kRootNodes) word(Y::kRootNodes)[lane] = 0;
         __syncwarp();
         push_roots<TMAX - 1>(have, K0, C, W, R, H);
         __syncwarp();
@@ -347,10 +353,19 @@ struct Tail {
         return (H >> hbit(ex, es)) & 1 ? n : n + n;
     }
 
+    __device__ __forceinline__ void count_nodes(int slot, int n, uint32_t &nodes) const {
+        if constexpr (kRootNodes) {
+            if (n) atomicAdd(word(Y::kRootNodes) + slot, uint32_t(n));
+        } else {
+            nodes += n;
+        }
+    }
+
     // Level K of a descent: idle lanes take frames, every lane takes its
-    // frame's next candidate and queues the rest (twice, so that lanes still
-    // idle share the candidates of frames just taken: 28 of 32 lanes busy
-    // instead of 20 on 7x7 roots); then the candidates are placed, and the
+    // frame's next candidate and queues the rest (up to three times, so that
+    // lanes still idle share the candidates of frames just taken: of 32 lanes
+    // 21, 26 and 28 busy after one, two and three turns on 7x7 roots; 50,000 7x7
+    // cases 890, 832 and 824 ms); then the candidates are placed, and the
     // placed cells' frames go on to the next level.
     template <int K>
     __device__ __forceinline__ void levels(int start, uint32_t &C, uint32_t (&W)[TMAX],
@@ -360,7 +375,7 @@ struct Tail {
             if (K <= start) {
                 uint32_t bt = 0;
 #pragma unroll 1
-                for (int turn = 0; turn < 2; ++turn) {
+                for (int turn = 0; turn < 3; ++turn) {
                     if (cnt[K] > 0) refill<K>(C, W, b, R, H);
                     const uint32_t rest = bt ? 0 : C & (C - 1);
                     if (!bt) bt = C & (0u - C);
@@ -404,7 +419,7 @@ struct Tail {
                         // to its first cell.
                         next &= kSym || es <= int(info >> 8) ? side_of : ~0u;
                     }
-                    if (K >= 2 || !kSym) nodes += __popc(next);
+                    if (K >= 2 || (!kSym && (info & 2))) count_nodes(slot, __popc(next), nodes);
                     next &= ~(info & 1);
                     if (K == 1) {
                         if (next) atomicAdd(word(Y::kAcc) + slot, uint32_t(__popc(next)));
@@ -439,12 +454,13 @@ struct Tail {
     }
 };
 
-// Row counting of the persistent kernels.  Frames that make a level full, lanes
-// at the row that start a count, and the bookkeeping rounds that a count
-// stands for (50,000 7x7 cases: 1,216 ms with 16 / 24 / 16; fill 10: 1,312,
-// fill 24: 1,257; roots 18: 1,294, roots 28: 1,189; rounds 32: 1,232, rounds 8:
-// 1,206).
-constexpr int kTailFill = 16;
+// Row counting of the persistent kernels.  Frames that make a level full
+// (squares, Lunnon rows), lanes at the row that start a count, and the
+// bookkeeping rounds that a count stands for (50,000 7x7 cases: 1,216 ms with
+// 16 / 24 / 16; fill 10: 1,312, fill 20: 904 against 832 at a later state, a CTA
+// less fitting on an SM; roots 18: 1,294, roots 28: 1,189; rounds 32: 1,232,
+// rounds 8: 1,206.  6x6 to depth 18: 116.6 ms with fill 16, 113.4 with 20).
+constexpr int kTailFill = 16, kLunnonTailFill = 20;
 constexpr int kTailRoots = 28;
 constexpr uint32_t kTailRounds = 8;
 // Levels above the row from which a subtree may be handed out: below, an item
