@@ -66,7 +66,7 @@ struct Progress {
 };
 
 // The reference's progress thread (sym_fold.cpp:442-454 materialized,
-// :574-589 streaming): a line after 5 s, then every half second while the
+// :574-589 streaming): a line after 5 s, then five a second while the
 // count runs (the reference: every 5 s; a whole 7x7 count takes 8), none after.
 class ProgressPrinter {
   public:
@@ -87,7 +87,7 @@ class ProgressPrinter {
         std::chrono::milliseconds wait(5000);
         while (!done_) {
             if (cv_.wait_for(lock, wait, [this] { return done_; })) break;
-            wait = std::chrono::milliseconds(500);
+            wait = std::chrono::milliseconds(200);
             const unsigned long long c = p_.completed.load();
             const double el = since(start_);
             const double rate = el > 0.0 ? double(c) / el : 0.0;

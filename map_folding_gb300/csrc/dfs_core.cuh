@@ -753,6 +753,9 @@ struct HeaderView {
 // every attempt stops the warp for two trips to L2 (500 7x7 cases: 30.8 ms with
 // 1, 29.1 with 16; 6x6: 135 and 131 ms).
 constexpr int kTakeLanes = 16;
+// What an idle warp waits for and takes: its lanes share from there (300 9x9 cases:
+// 41 ms with 32, 37 with 8 or 4, 40 with 2).
+constexpr int kWarpTake = 8;
 // Split items start at least this high above the counted level where no row is
 // counted by itself.
 constexpr int kMinRingHeight = 6;
@@ -769,7 +772,7 @@ __device__ __forceinline__ int split_quota(const HeaderView &now, unsigned long 
     queued = init >= num ? items : 0;
     const long long want = waiting - items;
     if (init < num || want <= 0) return 0;
-    const long long givers = (long long)warps - waiting / 32;
+    const long long givers = (long long)warps - waiting / kWarpTake;
     const long long q = givers > 0 ? (2 * want + givers - 1) / givers : 32;
     return q < 32 ? int(q) : 32;
 }

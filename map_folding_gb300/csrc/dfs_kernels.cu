@@ -458,13 +458,13 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             finished = 0;
             if (lane == 0) {
                 if (f) atomicAdd(&Q.hdr->completed, f);
-                if (reported_idle != 32) {
+                if (reported_idle != kWarpTake) {
                     atomicAdd(reinterpret_cast<unsigned long long *>(&Q.hdr->idle_lanes),
-                              (unsigned long long)(long long)(32 - reported_idle));
-                    reported_idle = 32;
+                              (unsigned long long)(long long)(kWarpTake - reported_idle));
+                    reported_idle = kWarpTake;
                 }
             }
-            const unsigned need = __ballot_sync(kFull, pre_stage == 0);
+            const unsigned need = __ballot_sync(kFull, pre_stage == 0 && lane < kWarpTake);
             const HeaderView now(Q.hdr);
             if (need && now.spawn_tail() != now.spawn_head()) take_splits(need);
             // A lane still holding a prefetched unit keeps the warp alive.

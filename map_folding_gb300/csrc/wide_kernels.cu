@@ -501,13 +501,13 @@ __global__ void __launch_bounds__(TPB)
             finished = 0;
             if (lane == 0) {
                 if (f) atomicAdd(&Q.hdr->completed, f);
-                if (reported_idle != 32) {
+                if (reported_idle != kWarpTake) {
                     atomicAdd(reinterpret_cast<unsigned long long *>(&Q.hdr->idle_lanes),
-                              (unsigned long long)(long long)(32 - reported_idle));
-                    reported_idle = 32;
+                              (unsigned long long)(long long)(kWarpTake - reported_idle));
+                    reported_idle = kWarpTake;
                 }
             }
-            const unsigned need = __ballot_sync(kFull, !init_left);
+            const unsigned need = __ballot_sync(kFull, !init_left && lane < kWarpTake);
             const HeaderView now(Q.hdr);
             if (need && now.spawn_tail() != now.spawn_head()) take_splits(need);
             if (__any_sync(kFull, busy) || __any_sync(kFull, init_left)) {
