@@ -15,8 +15,10 @@
 //   LunnonRules  -- mf.c:88-124 as a bitwise AND of per-dimension walk masks
 //   SymRules     -- sym_fold.cpp:179-204 (get_good)
 // Kernels:
-//   *_plain_kernel    one thread per unit (prefix state / case), one launch
-//   *_batched_kernel  persistent grid, device work queue, subtree splitting
+//   *_plain_kernel    one unit (prefix state / case) per lane, lanes of a warp
+//                     sharing what is left, one launch
+//   *_batched_kernel  persistent grid, device work queue, subtree splitting;
+//                     the last row counted on masks (tail.cuh)
 //
 // Every unit's list is checked to be a permutation of its placed items before
 // its search starts, which bounds every walk (see list_valid); the device
@@ -132,7 +134,9 @@ __global__ void launch_init_kernel(Queue Q, unsigned long long *counts, unsigned
     if (at < 32) reinterpret_cast<unsigned long long *>(Q.hdr)[at] = 0;  // its 256 bytes
 }
 
-constexpr int kRowLevels = 4;  // Lunnon: levels to go, of a map with rows, from which they pay
+// Lunnon: levels to go, of a map with rows, from which they pay (4x4 at depth 11,
+// four levels: 154 us by list, 81 by rows; below that a prefix is a node or two).
+constexpr int kRowLevels = 4;
 
 // Most cells of a list that the row count takes: all but two of a square's;
 // for Lunnon maps kRowLeaves' worth (what the frames' place holds as scratch).
@@ -181,7 +185,8 @@ struct LunnonSource {
 // a warp does its bookkeeping: it reports finished units and its idle-lane
 // count, lets idle lanes take split items, and -- while fewer split items are
 // queued than lanes wait for work -- lets a few busy lanes give away their
-// shallowest untried siblings.  A warp leaves when it is idle and all work is
+// shallowest untried siblings.  In between, lanes that run dry take pieces of
+// their own warp's work (share_in_warp).  A warp leaves when it is idle and all work is
 // accounted for, or when it has stayed idle for wait_limit rounds; leaving is
 // always safe, because the warp that owns a split item's parent keeps looping
 // until it has nothing left.  The last warp out checks that the work

@@ -2,9 +2,9 @@
 //
 // experiments/9x9/sym_fold9.cpp runs sym_fold's recursion with 128-bit masks
 // (sym_fold9.cpp:34, 261-312) so that cells past 63 can be counted.  This is
-// the same search as the 64-bit batched kernel -- lockstep rounds, the
-// unified page-start/step walk, a persistent grid fed by a warp-cooperative
-// split ring -- with 128-bit position masks, 96-cell successor lists and
+// the same search as the 64-bit batched kernel -- lockstep rounds, a persistent
+// grid fed by a warp-cooperative split ring, lanes sharing within the warp, the
+// last row counted on masks -- with 128-bit position masks, 96-cell successor lists and
 // 128-byte split records.  Cases arrive as the 64-byte records of the 64-bit
 // path (the host expands them to at most 64 cells); the list bytes past the
 // record start as zeros and are written by insertions before they are read.
