@@ -98,7 +98,8 @@ uint32_t mf_lunnon_state_stride(const mf_lunnon_plan *plan);
 int32_t mf_lunnon_collect(const mf_lunnon_plan *plan, int32_t depth, uint8_t *states,
                           uint64_t cap, uint64_t *count_out);
 
-/* Plain GPU DFS, one thread per prefix state, resumed at leaf start_leaf
+/* Plain GPU DFS, one lane per prefix state (lanes of a warp share what is left
+ * when theirs are done), resumed at leaf start_leaf
  * (= depth + 1) and stopped when the search returns to it.  d_per_state
  * (optional) receives each state's count; *d_total (optional) is ADDED to;
  * *d_nodes (optional) is added the number of leaf insertions the reference
@@ -196,7 +197,8 @@ uint32_t mf_sym_plan_case_bytes(const mf_sym_plan *plan);
 int32_t mf_sym_cases(const mf_sym_plan *plan, uint64_t start_case, uint64_t max_cases,
                      uint8_t *cycles, uint64_t *mults, uint64_t cap, uint64_t *count_out);
 
-/* Plain GPU count, one thread per case: d_counts[k] = completions of case k
+/* Plain GPU count, one lane per case (lanes of a warp share what is left when
+ * theirs are done): d_counts[k] = completions of case k
  * from cell start_i up to (excluding) stop_i, i.e. the number of distinct
  * cycles reaching stop_i cells (stop_i = n*n: complete foldings).  *d_nodes
  * (optional) is added the number of recurse_count calls (sym_fold.cpp:219).

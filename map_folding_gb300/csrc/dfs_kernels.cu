@@ -599,7 +599,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
 }
 
 template <int TPB, int LEVELS, int TMAX>
-__global__ void __launch_bounds__(TPB, TMAX > 0 ? 4 : 1)
+__global__ void __launch_bounds__(TPB, TMAX > 0 ? 4 : 768 / TPB)
     sym_batched_kernel(const uint8_t *__restrict__ edges, SymSource src, unsigned long long num,
                        unsigned long long *counts, unsigned long long *nodes_out, Queue Q,
                        uint32_t period, uint32_t wait_limit) {
@@ -864,9 +864,11 @@ cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int s
         return reset_queue(carve_queue(d_workspace, knobs.queue_capacity), d_counts, own_nodes, stream);
     cudaError_t e = cudaSuccess;
     const int sms = device_sm_count();
-    // The row count pays while a unit's search still enters the last row from
-    // above or near its start; a search to a partial depth has no last row.
-    const int row = stop_i == n * n && n >= 5 && start_i <= stop_i - n + 1 ? n : 0;
+    // The row count pays for units that end at the row or above it; a search to
+    // a partial depth has no last row.  100,000 units by list / by rows: 7x7 from
+    // 42 cells 0.86 / 0.28 ms, from 43 0.21 / 0.17; 8x8 from 56 0.46 / 0.27, from
+    // 57 0.13 / 0.21; 6x6 from 30 0.52 / 0.17, from 31 0.09 / 0.13.
+    const int row = stop_i == n * n && n >= 5 && start_i <= stop_i - n ? n : 0;
     const SymSource src{d_cycles, start_i, stop_i - 1, row};
     const int levels = pick_levels(stop_i - 1 - start_i, knobs.stack_mode == 1);
     const size_t tables = sym_tables_bytes(stop_i - start_i);
