@@ -385,7 +385,6 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
             }
             tail.enqueue_roots(ok, last - eval, c, W, r, h);
             tail.drain(none);
-            __syncwarp();
             if (ok) {
                 nodes += counted + tail.word(ServeTail::Y::kRootNodes)[lane];
                 leaves += tail.word(ServeTail::Y::kAcc)[lane];

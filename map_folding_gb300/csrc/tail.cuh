@@ -481,7 +481,9 @@ struct Tail {
         }
     }
 
-    // Count the queued frames to the end.
+    // Count the queued frames to the end.  A lane adds to other lanes' sums until
+    // it is through `last`, and reads other roots' tables there, so the lanes meet
+    // before any of them goes on to its own sum or to the next roots.
     __device__ __forceinline__ void drain(uint32_t &nodes) {
         for (;;) {
             int start = 0;
@@ -491,7 +493,10 @@ struct Tail {
 #pragma unroll
             for (int k = TMAX - 1; k >= 1; --k)
                 if (cnt[k] >= FILL) start = k;  // ... or the deepest full one
-            if (start == 0) return;
+            if (start == 0) {
+                __syncwarp();
+                return;
+            }
             uint32_t C = 0;
             Hist R = 0, H = 0;
             uint32_t W[TMAX] = {}, b[TMAX] = {};
