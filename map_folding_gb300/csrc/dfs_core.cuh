@@ -778,6 +778,18 @@ __device__ __forceinline__ int split_quota(const HeaderView &now, unsigned long 
     return q < 32 ? int(q) : 32;
 }
 
+// Report a warp's finished work items (all 32 lanes call).  A piece shared within
+// the warp takes one off its lane's count when it is made and, as every item,
+// adds one when it is done: a unit whose pieces still run is not in the sum, so
+// `completed` reaches the number of items only when nothing is left to do, and a
+// piece that got lost would show.  A sum below one waits on lane 0.
+__device__ __forceinline__ void report_finished(QueueHeader *hdr, long long &finished) {
+    const bool first = (threadIdx.x & 31) == 0;
+    const long long f = static_cast<long long>(warp_sum(static_cast<unsigned long long>(finished)));
+    finished = first && f < 0 ? f : 0;
+    if (first && f > 0) atomicAdd(&hdr->completed, static_cast<unsigned long long>(f));
+}
+
 // Called once per warp (lane 0) as it leaves a persistent launch, after all
 // of its counters are in.  Warps leave early on purpose (idle for wait_limit
 // rounds while others still work), so only the last warp out can tell

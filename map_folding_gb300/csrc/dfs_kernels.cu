@@ -208,13 +208,13 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
     const int lane = threadIdx.x & 31;
     const unsigned lt_mask = (1u << lane) - 1u;
     bool busy = false, fresh = false;
-    bool whole = true;     // a unit or split item, not a piece shared within the warp
     bool walking = false;  // a resumable walk is under way
     SymHopRules::Walk swalk{};
     LunnonRules::Walk lwalk{};
     int lvl = 0, root = 0, last = 0, eval = 0;
     uint32_t owner = 0;
-    unsigned long long leaves = 0, nodes = 0, finished = 0, started = 0;
+    unsigned long long leaves = 0, nodes = 0, started = 0;
+    long long finished = 0;  // items done less pieces taken, not reported yet
     uint32_t idle_rounds = 0, round = 0;
     int reported_idle = 0;  // lane 0: idle lanes this warp last reported
     bool ring_hint = false;  // warp-uniform: the split ring probably has items
@@ -269,7 +269,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             atomicAdd(counts + owner, leaves * weight);
         }
         leaves = 0;
-        if (whole) ++finished;
+        ++finished;
     };
 
     int row_len = 0;  // Lunnon: leaves of a row of the map
@@ -309,7 +309,6 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
             for (int k2 = 0; k2 < WORDS; ++k2) L.set_word(k2, w[k2]);
             owner = w[17];
             root = int(w[20]);
-            whole = true;
             if (kSym) {
                 last = sym.last;
                 S.base = sym.start_i;
@@ -360,8 +359,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         ring_put(Q, first + rank, w);
     };
 
-    // Pieces shared within the warp are no work items of their own: a piece
-    // belongs to its unit's count and to nobody's bookkeeping.
+    // Pieces shared within the warp are no items of the ring: they are added up
+    // within the warp, and its units count as finished when they are too.
     auto share = [&](unsigned idle) -> bool {
         uint32_t whose = 0;
         int its_row = 0;
@@ -384,7 +383,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                 }
                 S.set(root, mask);
                 eval = advance(L, S, lvl, root);
-                whole = false;
+                --finished;  // see report_finished
                 walking = false;
                 by_walk = false;
                 fresh = false;
@@ -407,7 +406,6 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                         if (4 * q + k < WORDS) L.set_word(4 * q + k, ws[k]);
                 }
                 ++started;
-                whole = true;
                 bool ok;
                 if (kSym) {
                     owner = uint32_t(pre_k);
@@ -459,10 +457,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         const bool bookkeeping = ++round >= period;
         if (!__any_sync(kFull, busy)) {
             // The whole warp is idle: report, look for split items, decide.
-            const unsigned long long f = warp_sum(finished);
-            finished = 0;
+            report_finished(Q.hdr, finished);
             if (lane == 0) {
-                if (f) atomicAdd(&Q.hdr->completed, f);
                 if (reported_idle != kWarpTake) {
                     atomicAdd(reinterpret_cast<unsigned long long *>(&Q.hdr->idle_lanes),
                               (unsigned long long)(long long)(kWarpTake - reported_idle));
@@ -564,11 +560,9 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         if (!bookkeeping) continue;
         round = 0;
         const unsigned idle_mask = __ballot_sync(kFull, !busy);
-        const unsigned long long f = warp_sum(finished);
-        finished = 0;
+        report_finished(Q.hdr, finished);
         long long queued = 0;
         if (lane == 0) {
-            if (f) atomicAdd(&Q.hdr->completed, f);
             const int idle_now = __popc(idle_mask);
             if (idle_now != reported_idle) {
                 atomicAdd(reinterpret_cast<unsigned long long *>(&Q.hdr->idle_lanes),
@@ -617,9 +611,11 @@ __global__ void __launch_bounds__(TPB, TMAX > 0 ? 4 : 768 / TPB)
 }
 
 // Shared memory: the maps' neighbour tables and their instance records
-// (meta_bytes in all, records at inst_offset), then the carve.
+// (meta_bytes in all, records at inst_offset), then the carve.  One CTA of 512
+// threads fits on an SM by shared memory, so it may take the registers of one
+// (left to the compiler: 64, and 56 bytes spilled).
 template <int TPB, int LEVELS, int TMAX>
-__global__ void __launch_bounds__(TPB)
+__global__ void __launch_bounds__(TPB, TPB == 512 ? 1 : 0)
     lunnon_batched_kernel(const uint8_t *__restrict__ meta, uint32_t meta_bytes,
                           uint32_t inst_offset, LunnonSource src, unsigned long long num,
                           unsigned long long *counts, unsigned long long *nodes_out, Queue Q,

@@ -303,7 +303,7 @@ __global__ void __launch_bounds__(TPB)
     if constexpr (kRow) pages = sym_row_pages(smem, last, kWideCells);
     const int row_first = last + 1 - kWideRow;  // first level of the counted row
     int row_level = kNoRow;                     // ... of the unit at hand
-    bool by_walk = false, whole = true, share_miss = false;
+    bool by_walk = false, share_miss = false;
     const unsigned lt_mask = (1u << lane) - 1u;
     constexpr int kOwner = kWideWords, kMaskW = kWideWords + 1, kRoot = kWideWords + 5,
                   kRowOk = kWideWords + 6;
@@ -313,7 +313,8 @@ __global__ void __launch_bounds__(TPB)
     bool init_left = (unsigned long long)lane * warps < num;
     int lvl = start_i, root = start_i, eval = start_i;
     uint32_t owner = 0;
-    unsigned long long leaves = 0, nodes = 0, finished = 0, started = 0;
+    unsigned long long leaves = 0, nodes = 0, started = 0;
+    long long finished = 0;  // items done less pieces taken, not reported yet
     uint32_t idle_rounds = 0, round = 0, nap = 256;
     int reported_idle = 0;
     bool ring_hint = false;
@@ -321,7 +322,7 @@ __global__ void __launch_bounds__(TPB)
     auto flush = [&]() {
         if (leaves) atomicAdd(counts + owner, leaves);
         leaves = 0;
-        if (whole) ++finished;
+        ++finished;
     };
 
     auto take_splits = [&](unsigned need) -> bool {
@@ -342,7 +343,6 @@ __global__ void __launch_bounds__(TPB)
                                 uint64_t(w[kMaskW + 2]) | (uint64_t(w[kMaskW + 3]) << 32)});
             eval = advance_w(L, S, lvl, root);  // an item's mask is never empty
             fresh = false;
-            whole = true;
             by_walk = false;
             if (kRow) row_level = w[kRowOk] ? row_first : kNoRow;
             busy = eval >= 0;
@@ -420,7 +420,7 @@ __global__ void __launch_bounds__(TPB)
             lvl = level;
             S.set(root, mask);
             eval = advance_w(L, S, lvl, root);
-            whole = false;
+            --finished;  // see report_finished
             fresh = false;
             by_walk = false;
             busy = true;
@@ -465,7 +465,6 @@ __global__ void __launch_bounds__(TPB)
                     owner = uint32_t(k);
                     root = start_i;
                     ++started;
-                    whole = true;
                     by_walk = false;
                     const bool ok = list_valid(L, start_i);
                     if (kRow)
@@ -497,10 +496,8 @@ __global__ void __launch_bounds__(TPB)
         }
         const bool bookkeeping = ++round >= period;
         if (!__any_sync(kFull, busy)) {
-            const unsigned long long f = warp_sum(finished);
-            finished = 0;
+            report_finished(Q.hdr, finished);
             if (lane == 0) {
-                if (f) atomicAdd(&Q.hdr->completed, f);
                 if (reported_idle != kWarpTake) {
                     atomicAdd(reinterpret_cast<unsigned long long *>(&Q.hdr->idle_lanes),
                               (unsigned long long)(long long)(kWarpTake - reported_idle));
@@ -570,10 +567,8 @@ __global__ void __launch_bounds__(TPB)
         if (!bookkeeping) continue;
         round = 0;
         const unsigned idle_mask = __ballot_sync(kFull, !busy);
-        const unsigned long long f = warp_sum(finished);
-        finished = 0;
+        report_finished(Q.hdr, finished);
         if (lane == 0) {
-            if (f) atomicAdd(&Q.hdr->completed, f);
             const int idle_now = __popc(idle_mask);
             if (idle_now != reported_idle) {
                 atomicAdd(reinterpret_cast<unsigned long long *>(&Q.hdr->idle_lanes),

@@ -218,3 +218,22 @@ def test_9x9_rows(host, start):
         got, nodes, _ = _wide(host, edges, start, cases, 1, rows)
         assert list(got) == [l for l, _ in want]
         assert nodes == sum(k for _, k in want)
+
+
+@pytest.mark.parametrize("seed", range(8))
+@pytest.mark.parametrize("kind", ["square", "map", "strip", "9x9"])
+def test_warps_stay_until_shared_pieces_are_done(host, orc, kind, seed):
+    """No warp goes home while a piece shared within another still runs: all is
+    counted when the first one leaves."""
+    if kind == "square":
+        edges, cases = _sym_cases(orc, 5, 13, 1, seed)
+        got, _, left = _sym(host, edges, 5, 13, cases, seed)
+    elif kind == "9x9":
+        edges, rng = _edges9(host), np.random.default_rng(seed)
+        cases = np.array([_descend(edges, 56, rng, back=30)])
+        got, _, left = _wide(host, edges, 56, cases, seed)
+    else:
+        dims, depth = {"map": ((5, 4), 9), "strip": ((1, 14), 5)}[kind]
+        _, b, _ = orc.lunnon_collect(dims, depth)
+        got, _, left = _lunnon(host, [(dims, depth, b[seed:seed + 1])], seed)
+    assert left == got.sum()
