@@ -66,8 +66,8 @@ struct Progress {
 };
 
 // The reference's progress thread (sym_fold.cpp:442-454 materialized,
-// :574-589 streaming): a line after 5 s, then five a second while the
-// count runs (the reference: every 5 s; a whole 7x7 count takes 8), none after.
+// :574-589 streaming): a line every 5 s while the count runs and, after any of
+// these, one as it ends.
 class ProgressPrinter {
   public:
     ProgressPrinter(const Progress &p, bool stream, unsigned long long planned)
@@ -84,10 +84,8 @@ class ProgressPrinter {
   private:
     void run() {
         std::unique_lock<std::mutex> lock(mu_);
-        std::chrono::milliseconds wait(5000);
-        while (!done_) {
-            if (cv_.wait_for(lock, wait, [this] { return done_; })) break;
-            wait = std::chrono::milliseconds(200);
+        for (bool first = true; !done_; first = false) {
+            if (cv_.wait_for(lock, std::chrono::seconds(5), [this] { return done_; }) && first) break;
             const unsigned long long c = p_.completed.load();
             const double el = since(start_);
             const double rate = el > 0.0 ? double(c) / el : 0.0;
