@@ -542,10 +542,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                     }
                 }
                 tail.enqueue_roots(ok, K0, C, W, R, H);
-                tail.drain(counted);
-                nodes += counted;
+                tail.drain(counted, leaves, nodes);
                 if (ok) {
-                    leaves += tail.word(RowTail::Y::kAcc)[lane];
                     eval = apply_advance(L, S, lvl, eval, root, last, fresh, 0, leaves);
                     fresh = false;
                     if (eval < 0) {

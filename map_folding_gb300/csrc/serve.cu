@@ -366,7 +366,7 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
         const unsigned at = __ballot_sync(kFull, here);
         if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
             uint32_t W[ServeTail::kRow] = {};
-            uint32_t c = 0, counted = 0, none = 0;
+            uint32_t c = 0, counted = 0;
             ServeTail::Hist r = 0, h = 0;
             bool ok = false;
             tail.prepare_setup();
@@ -384,10 +384,8 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
                 }
             }
             tail.enqueue_roots(ok, last - eval, c, W, r, h);
-            tail.drain(none);
+            tail.drain(counted, leaves, nodes);
             if (ok) {
-                nodes += counted + tail.word(ServeTail::Y::kRootNodes)[lane];
-                leaves += tail.word(ServeTail::Y::kAcc)[lane];
                 eval = apply_advance(L, S, lvl, eval, root, last, fresh, 0, leaves);
                 fresh = false;
                 if (eval < 0) {

@@ -108,11 +108,54 @@ struct HistWord<true> {
     using type = uint64_t;
 };
 
+// Most ways to place t row cells into 31 gaps so that their arcs to the row before
+// cross nowhere, whatever the list (a bound).  The first arc cuts the gaps, its own
+// in two, and the other cells between its sides; as its end goes through the gaps
+// in order, cells only ever pass from one side to the other.
+constexpr uint64_t most_rows(int t) {
+    uint64_t g[10][32] = {};
+    for (int n = 0; n < 32; ++n) g[0][n] = 1;
+    for (int k = 1; k <= t; ++k)
+        for (int n = 1; n < 32; ++n) {
+            uint64_t best[10] = {};
+            for (int p = 1; p <= n; ++p) {
+                uint64_t most = 0;
+                for (int j = 0; j < k; ++j) {
+                    if (best[j] > most) most = best[j];
+                    best[j] = most + g[j][p] * g[k - 1 - j][n + 1 - p];
+                }
+            }
+            for (int j = 0; j < k; ++j)
+                if (best[j] > g[k][n]) g[k][n] = best[j];
+        }
+    return g[t][31];
+}
+
+// Whether 32 bits hold a count's sums whatever the roots: a root's leaves in kAcc,
+// and all 32 roots' nodes in one lane (a square's last cells are no nodes).  They
+// do for rows of up to seven (410,013,942 leaves, 1,308,637,184 nodes); 9x9 rows
+// could have 3.7e10 leaves by this bound.
+constexpr bool sums_fit(int t, bool square) {
+    uint64_t nodes = 1;
+    for (int k = 1; k <= t - square; ++k) nodes += most_rows(k);
+    return most_rows(t) < (1ULL << 32) && 32 * nodes < (1ULL << 32);
+}
+static_assert(sums_fit(7, true) && sums_fit(6, false) && !sums_fit(8, true), "sums of a row count");
+
+// Elsewhere the sums go to 64-bit ones once a lane (or root, see kRootNodes) has
+// counted this many nodes.  A turn adds at most 31 nodes a level and 31 x 31 at the
+// last, 32 lanes' to a root, and at most 31 leaves a node.  (2,000 8x8 cases 58.8 ms
+// without, 58.5 with; with the 64-bit sums inside the loop 59.4, and 5,000 7x7 cases
+// 2.5 % longer.)
+constexpr uint32_t kTailNodes = 1 << 21;
+static_assert(uint64_t(kTailNodes + 31 + 7 * 31 + 31 * 31) * 31 * 32 < (1ULL << 32), "sums of a row count");
+
 // With kRootNodes the nodes too are added up per root, not per lane.
 template <bool kSym, int TMAX, int CELLS, int FILL, int BITS = 5, bool kRootNodes = false>
 struct Tail {
     using Y = TailLayout<TMAX, CELLS, FILL, BITS>;
     static constexpr int kRow = TMAX;
+    static constexpr bool kLong = kRootNodes || !sums_fit(TMAX, kSym);
     // R: the gap numbers of the earlier picks, five bits each, the latest
     // lowest; H: the h bits, and the root's slot above them.
     using Hist = typename HistWord<(TMAX > 8)>::type;
@@ -481,10 +524,35 @@ struct Tail {
         }
     }
 
-    // Count the queued frames to the end.  A lane adds to other lanes' sums until
-    // it is through `last`, and reads other roots' tables there, so the lanes meet
-    // before any of them goes on to its own sum or to the next roots.
-    __device__ __forceinline__ void drain(uint32_t &nodes) {
+    // Take the 32-bit sums (this lane's nodes, its root's leaves and nodes) to
+    // the caller's (all lanes call).  A lane adds to other lanes' sums until it is
+    // through `last`, and reads other roots' tables there, so the lanes meet first.
+    __device__ __forceinline__ void collect(uint32_t &counted, unsigned long long &leaves,
+                                            unsigned long long &nodes) const {
+        __syncwarp();
+        leaves += word(Y::kAcc)[lane];
+        nodes += counted;
+        counted = 0;
+        if (kRootNodes) nodes += word(Y::kRootNodes)[lane];
+    }
+
+    // Count the queued frames to the end: the leaves of the lane's root are added
+    // to `leaves`, `counted` and the nodes to `nodes`.
+    __device__ __forceinline__ void drain(uint32_t counted, unsigned long long &leaves,
+                                          unsigned long long &nodes) {
+        for (bool more = true; more;) {
+            more = run(counted);
+            collect(counted, leaves, nodes);
+            if (more) {
+                word(Y::kAcc)[lane] = 0;
+                if (kRootNodes) word(Y::kRootNodes)[lane] = 0;
+                __syncwarp();
+            }
+        }
+    }
+
+    // Count queued frames until none is left, or (true) the sums must be taken over.
+    __device__ __forceinline__ bool run(uint32_t &nodes) {
         for (;;) {
             int start = 0;
 #pragma unroll
@@ -493,14 +561,13 @@ struct Tail {
 #pragma unroll
             for (int k = TMAX - 1; k >= 1; --k)
                 if (cnt[k] >= FILL) start = k;  // ... or the deepest full one
-            if (start == 0) {
-                __syncwarp();
-                return;
-            }
+            if (start == 0) return false;
             uint32_t C = 0;
             Hist R = 0, H = 0;
             uint32_t W[TMAX] = {}, b[TMAX] = {};
             levels<TMAX - 1>(start, C, W, b, R, H, nodes);
+            if (kLong && __any_sync(kFull, (kRootNodes ? word(Y::kRootNodes)[lane] : nodes) >= kTailNodes))
+                return true;
         }
     }
 };

@@ -549,10 +549,8 @@ __global__ void __launch_bounds__(TPB)
                     else by_walk = true;
                 }
                 tail.enqueue_roots(ok, last - eval, c, W, r, h);
-                tail.drain(counted);
-                nodes += counted;
+                tail.drain(counted, leaves, nodes);
                 if (ok) {
-                    leaves += tail.word(WideTail::Y::kAcc)[lane];
                     eval = apply_advance_w(L, S, lvl, eval, root, last, fresh, Mask128{0, 0}, leaves);
                     fresh = false;
                     if (eval < 0) {

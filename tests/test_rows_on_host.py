@@ -19,16 +19,15 @@ def _cut(text, begin, end):
     return text[at:text.index(end, at)]
 
 
-@pytest.fixture(scope="module")
-def host(tmp_path_factory):
-    d = tmp_path_factory.mktemp("rows")
+def _build(d, change=lambda name, text: text):
+    """The kernels' device code as a host library; change(file, text) may edit it."""
     src = d / "pkg" / "csrc"
     src.mkdir(parents=True)
     shutil.copytree(HERE.parent / "include", d / "include")
     for f in (*CSRC.glob("*.cuh"), *CSRC.glob("*.hpp"), *CSRC.glob("*.inl")):
         text = f.read_text()
         text = re.sub(r'asm\("shl\.b(\d+).*"r"\((\w)\)\);', r"r = \2 < \1 ? decltype(r)(1) << \2 : 0;", text)
-        (src / f.name).write_text(text)
+        (src / f.name).write_text(change(f.name, text))
     loop = _cut((CSRC / "dfs_kernels.cu").read_text(), "// Lunnon: levels to go",
                 "template <int TPB, int LEVELS, int TMAX>\n__global__")
     (src / "persistent.inc").write_text(
@@ -43,6 +42,11 @@ def host(tmp_path_factory):
                     "-I", str(HERE / "host"), "-I", str(src), str(HERE / "host" / "rows.cpp"),
                     str(src / "host.cpp"), "-o", str(lib), "-pthread"], check=True)
     return ctypes.CDLL(str(lib))
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    return _build(tmp_path_factory.mktemp("rows"))
 
 
 def _ptr(a):
@@ -237,3 +241,19 @@ def test_warps_stay_until_shared_pieces_are_done(host, orc, kind, seed):
         _, b, _ = orc.lunnon_collect(dims, depth)
         got, _, left = _lunnon(host, [(dims, depth, b[seed:seed + 1])], seed)
     assert left == got.sum()
+
+
+def test_long_counts_go_on_in_64_bits(tmp_path, orc):
+    """Where a row count's 32-bit sums might not do they are taken over in time;
+    here as soon as anything has been counted, on rows of eight and nine."""
+    def at_once(name, text):
+        if name != "tail.cuh":
+            return text
+        assert text.count("kTailNodes = 1 << 21;") == 1
+        return text.replace("kTailNodes = 1 << 21;", "kTailNodes = 1;")
+
+    host = _build(tmp_path, at_once)
+    test_square_rows(host, orc, 8, 54, 40, 1)
+    test_square_rows(host, orc, 8, 57, 40, 2)
+    test_9x9_rows(host, 70)
+    test_9x9_rows(host, 74)
