@@ -761,6 +761,15 @@ constexpr int kWarpTake = 8;
 // 230 us, 2x10 at 12 448 / 425 us).
 constexpr int kMinRingHeight = 6;
 
+// Square units of at most kShallow levels searched by list are spread over ten warps
+// an SM and no more: a warp runs as long as its longest unit, so fuller warps take
+// fewer instructions in all, and ten an SM cover the latencies (100,000 7x7 units
+// from 44 cells: 118.8 us with the first warps full, 152.4 spread over all 24 an SM,
+// 110.5 over ten; 2,000: 77, 60, 60; of 8 levels 100,000 and 12,000: 716, 647, 550
+// and 535, 289, 277; of 9 on 8x8, 12,000: 1,442, 574, 581).
+constexpr int kShallow = 7;
+constexpr int kShallowWarps = 10;
+
 // How many split items a warp with work is to give now, of a launch of `num`
 // units and `warps` warps: its share of what is wanted, twice over.  Every
 // such warp sees the same number, and if all gave all they could the ring

@@ -202,7 +202,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                                                 unsigned long long num,
                                                 unsigned long long *counts,
                                                 unsigned long long *nodes_out, const Queue &Q,
-                                                uint32_t period, uint32_t wait_limit,
+                                                uint32_t period, uint32_t wait_limit, uint32_t spread,
                                                 const List<TPB> &L, Stk &S, uint8_t *tail_area) {
     constexpr int kVecs = (WORDS + 3) / 4;
     const int lane = threadIdx.x & 31;
@@ -238,11 +238,10 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
     }
 
     // Prefetch state: 0 = no initial unit left for this lane, 1 = index
-    // taken.  The first indices come from one warp-aggregated atomicAdd; with
-    // fewer units than lanes every warp takes its share of them, not the
-    // first warps 32 each.
+    // taken.  The first indices come from one warp-aggregated atomicAdd; fewer
+    // units than lanes are spread over `spread` warps.
     const unsigned long long warps = (unsigned long long)gridDim.x * (TPB / 32);
-    const unsigned long long even = (num + warps - 1) / warps;
+    const unsigned long long even = (num + spread - 1) / spread;
     const int own = even < 32 ? int(even) : 32;
     unsigned long long pre_k = 0;
     {
@@ -594,7 +593,7 @@ template <int TPB, int LEVELS, int TMAX>
 __global__ void __launch_bounds__(TPB, TMAX > 0 ? 4 : 768 / TPB)
     sym_batched_kernel(const uint8_t *__restrict__ edges, SymSource src, unsigned long long num,
                        unsigned long long *counts, unsigned long long *nodes_out, Queue Q,
-                       uint32_t period, uint32_t wait_limit) {
+                       uint32_t period, uint32_t wait_limit, uint32_t spread) {
     extern __shared__ __align__(16) uint8_t smem[];
     using C = Carve<TPB, 16, LEVELS>;
     stage_sym_hop_rules<TPB>(smem, edges, src.start_i, src.last - src.start_i + 1);
@@ -604,7 +603,7 @@ __global__ void __launch_bounds__(TPB, TMAX > 0 ? 4 : 768 / TPB)
     init_stack<TPB, 16, LEVELS>(S, smem, tables);
     LunnonSource none{};
     persistent_loop<TPB, 16, true, TMAX>(smem, nullptr, src, none, num, counts, nodes_out, Q, period,
-                                         wait_limit, L, S,
+                                         wait_limit, spread, L, S,
                                          tail_of_warp<true, TMAX>(smem + tables + C::kThreadBytes));
 }
 
@@ -617,7 +616,7 @@ __global__ void __launch_bounds__(TPB, TPB == 512 ? 1 : 0)
     lunnon_batched_kernel(const uint8_t *__restrict__ meta, uint32_t meta_bytes,
                           uint32_t inst_offset, LunnonSource src, unsigned long long num,
                           unsigned long long *counts, unsigned long long *nodes_out, Queue Q,
-                          uint32_t period, uint32_t wait_limit) {
+                          uint32_t period, uint32_t wait_limit, uint32_t spread) {
     extern __shared__ __align__(16) uint8_t smem[];
     using C = Carve<TPB, 17, LEVELS>;
     for (uint32_t k = threadIdx.x; k < meta_bytes / 4; k += TPB)
@@ -629,7 +628,7 @@ __global__ void __launch_bounds__(TPB, TPB == 512 ? 1 : 0)
     SymSource none{};
     persistent_loop<TPB, 17, false, TMAX>(
         smem, reinterpret_cast<const LunnonInstanceDev *>(smem + inst_offset), none, src, num, counts,
-        nodes_out, Q, period, wait_limit, L, S,
+        nodes_out, Q, period, wait_limit, spread, L, S,
         tail_of_warp<false, TMAX>(smem + meta_bytes + C::kThreadBytes));
 }
 
@@ -750,19 +749,23 @@ __global__ void phantom_ticket_kernel(QueueHeader *hdr) { hdr->spawn_tail = 1; }
 struct LaunchShape {
     unsigned blocks;
     uint64_t ring;
+    uint32_t spread;  // warps that fewer units than lanes are spread over
 };
 
 LaunchShape persistent_shape(int sms, int bpsm, int tpb, uint64_t units, int levels,
-                             uint64_t ring_knob) {
+                             uint64_t ring_knob, bool square_list = false) {
     const uint64_t full = uint64_t(sms) * uint64_t(bpsm);
-    if (levels > 10) return LaunchShape{unsigned(full), ring_knob};
+    if (levels > 10) return LaunchShape{unsigned(full), ring_knob, uint32_t(full * (tpb / 32))};
     const uint64_t warps = (units + 3) / 4;
     const uint64_t per_block = uint64_t(tpb / 32);
     uint64_t blocks = (warps + per_block - 1) / per_block;
     blocks = blocks < 1 ? 1 : (blocks > full ? full : blocks);
     uint64_t ring = 1024;
     while (ring < 2 * blocks * uint64_t(tpb) && ring < ring_knob) ring <<= 1;
-    return LaunchShape{unsigned(blocks), ring < ring_knob ? ring : ring_knob};
+    uint64_t spread = blocks * per_block;
+    if (square_list && levels <= kShallow && spread > uint64_t(sms) * kShallowWarps)
+        spread = uint64_t(sms) * kShallowWarps;
+    return LaunchShape{unsigned(blocks), ring < ring_knob ? ring : ring_knob, uint32_t(spread)};
 }
 
 cudaError_t reset_queue(const Queue &Q, uint64_t *counts, uint64_t words, cudaStream_t stream) {
@@ -875,12 +878,14 @@ cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int s
         e = prepare(sym_batched_kernel<TPB, LV, TM>, smem, TPB, knobs.blocks_per_sm, bpsm);      \
         if (e != cudaSuccess) return e;                                                          \
         const LaunchShape shape =                                                                \
-            persistent_shape(sms, bpsm, TPB, num, stop_i - start_i, knobs.queue_capacity);       \
+            persistent_shape(sms, bpsm, TPB, num, stop_i - start_i, knobs.queue_capacity,        \
+                             TM == 0);                                                           \
         const Queue Q = carve_queue(d_workspace, shape.ring);                                    \
         e = reset_queue(Q, d_counts, num + own_nodes, stream);                                   \
         if (e != cudaSuccess) return e;                                                          \
         sym_batched_kernel<TPB, LV, TM><<<shape.blocks, TPB, smem, stream>>>(                    \
-            d_edges, src, num, counts, nodes, Q, knobs.node_budget, knobs.wait_limit);          \
+            d_edges, src, num, counts, nodes, Q, knobs.node_budget, knobs.wait_limit,           \
+            shape.spread);                                                                       \
     } while (0)
     if (row == 8) {
         MF_SYM_BATCHED(128, 0, 8);
@@ -938,7 +943,7 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
         if (e != cudaSuccess) return e;                                                          \
         lunnon_batched_kernel<TPB, LV, TM><<<shape.blocks, TPB, smem, stream>>>(                 \
             d_meta, mb, inst_offset, src, num, counts, nodes, Q, knobs.node_budget,             \
-            knobs.wait_limit);                                                                   \
+            knobs.wait_limit, shape.spread);                                                     \
     } while (0)
     if (row_levels >= kRowLevels) {
         // All the maps' tables are in every CTA's shared memory, so many small

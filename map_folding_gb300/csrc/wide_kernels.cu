@@ -10,6 +10,7 @@
 // record start as zeros and are written by insertions before they are read.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "dfs_core.cuh"
@@ -281,7 +282,7 @@ __global__ void __launch_bounds__(TPB)
     sym_wide_kernel(const uint8_t *__restrict__ edges, int start_i, int last,
                     const uint8_t *__restrict__ cycles, uint32_t record_bytes, unsigned long long num,
                     unsigned long long *counts, unsigned long long *nodes_out, Queue Q,
-                    uint4 *slots, uint32_t period, uint32_t wait_limit) {
+                    uint4 *slots, uint32_t period, uint32_t wait_limit, uint32_t spread) {
     extern __shared__ __align__(16) uint8_t smem[];
     stage_wide_tables<TPB>(smem, edges);
     __syncthreads();
@@ -307,10 +308,10 @@ __global__ void __launch_bounds__(TPB)
     const unsigned lt_mask = (1u << lane) - 1u;
     constexpr int kOwner = kWideWords, kMaskW = kWideWords + 1, kRoot = kWideWords + 5,
                   kRowOk = kWideWords + 6;
-    // With fewer units than lanes every warp takes its share of them.
+    // Fewer units than lanes are spread over `spread` warps.
     const unsigned long long warps = (unsigned long long)gridDim.x * (TPB / 32);
     bool busy = false, fresh = false;
-    bool init_left = (unsigned long long)lane * warps < num;
+    bool init_left = (unsigned long long)lane * spread < num;
     int lvl = start_i, root = start_i, eval = start_i;
     uint32_t owner = 0;
     unsigned long long leaves = 0, nodes = 0, started = 0;
@@ -627,11 +628,14 @@ cudaError_t launch_wide_levels(const uint8_t *d_edges, int start_i, int last, co
     if (e != cudaSuccess) return e;
     if (fit < 1) return cudaErrorInvalidConfiguration;
     if (knobs.blocks_per_sm > 0 && int(knobs.blocks_per_sm) < fit) fit = int(knobs.blocks_per_sm);
-    sym_wide_kernel<kWideTPB, LEVELS, kRow><<<unsigned(device_sm_count() * fit), kWideTPB, smem, stream>>>(
+    const int sms = device_sm_count();
+    uint32_t spread = uint32_t(sms * fit * (kWideTPB / 32));
+    if (!kRow && last + 1 - start_i <= kShallow) spread = std::min(spread, uint32_t(sms * kShallowWarps));
+    sym_wide_kernel<kWideTPB, LEVELS, kRow><<<unsigned(sms * fit), kWideTPB, smem, stream>>>(
         d_edges, start_i, last, d_cycles, record_bytes, num,
         reinterpret_cast<unsigned long long *>(d_counts),
         reinterpret_cast<unsigned long long *>(d_nodes), Q, slots, knobs.node_budget,
-        knobs.wait_limit);
+        knobs.wait_limit, spread);
     return cudaGetLastError();
 }
 

@@ -35,6 +35,7 @@ void watch(const QueueHeader &hdr, const uint64_t *counts, uint64_t num, uint64_
 
 using Ull = unsigned long long;
 constexpr uint32_t kPeriod = 64, kWaitLimit = 1u << 30;
+uint32_t g_spread;
 
 template <int TMAX>
 void run_sym(const uint8_t *edges, const SymSource &src, uint64_t num, uint64_t *counts,
@@ -50,9 +51,11 @@ void run_sym(const uint8_t *edges, const SymSource &src, uint64_t num, uint64_t 
         S.base = 0;
         persistent_loop<TPB, 16, true, TMAX>(
             smem, nullptr, src, LunnonSource{}, num, reinterpret_cast<Ull *>(counts),
-            reinterpret_cast<Ull *>(nodes), Q, kPeriod, kWaitLimit, L, S,
+            reinterpret_cast<Ull *>(nodes), Q, kPeriod, kWaitLimit,
+            g_spread, L, S,
             tail_of_warp<true, TMAX>(smem + tables + C::kThreadBytes));
     };
+    g_spread = 1 + seed % 4;
     host::launch(128, seed, [](void *f) { (*static_cast<decltype(body) *>(f))(); }, &body);
 }
 
@@ -71,8 +74,9 @@ void run_lunnon(const uint8_t *meta, uint32_t bytes, uint32_t inst_offset, const
         persistent_loop<TPB, 17, false, TMAX>(
             smem, reinterpret_cast<const LunnonInstanceDev *>(smem + inst_offset), SymSource{}, src,
             num, reinterpret_cast<Ull *>(counts), reinterpret_cast<Ull *>(nodes), Q, kPeriod,
-            kWaitLimit, L, S, tail_of_warp<false, TMAX>(smem + bytes + C::kThreadBytes));
+            kWaitLimit, g_spread, L, S, tail_of_warp<false, TMAX>(smem + bytes + C::kThreadBytes));
     };
+    g_spread = 1 + seed % 4;
     host::launch(128, seed, [](void *f) { (*static_cast<decltype(body) *>(f))(); }, &body);
 }
 
@@ -83,8 +87,10 @@ void run_wide(const uint8_t *edges, int start, const uint8_t *cycles, uint64_t n
     auto body = [&] {
         sym_wide_kernel<TPB, 56, kRow>(edges, start, 80, cycles, kWideCells, num,
                                        reinterpret_cast<Ull *>(counts),
-                                       reinterpret_cast<Ull *>(nodes), Q, slots, kPeriod, kWaitLimit);
+                                       reinterpret_cast<Ull *>(nodes), Q, slots, kPeriod, kWaitLimit,
+                                       g_spread);
     };
+    g_spread = 1 + seed % (TPB / 32);
     host::launch(TPB, seed, [](void *f) { (*static_cast<decltype(body) *>(f))(); }, &body);
 }
 

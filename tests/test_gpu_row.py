@@ -96,3 +96,20 @@ def test_cases_that_are_no_foldings(engine, cuda, n):
     want, want_nodes = _plain(engine, cuda, n, start, cases)
     assert (got == want).all()
     assert nodes == want_nodes
+
+
+@pytest.mark.parametrize("n,start", [(5, 21), (7, 44), (8, 58)])
+@pytest.mark.parametrize("num", [1, 31, 1519, 1521, 12000, 48641])
+def test_many_shallow_units(engine, cuda, orc, n, start, num):
+    """Units that end a few cells further, at the numbers where their spreading
+    over the warps changes."""
+    rng = np.random.default_rng([n, start])
+    root = np.zeros(64, np.uint8)
+    root[:3] = (1, 2, 0)
+    some = np.array([_descend(orc, n, root, 3, start, rng) for _ in range(37)])
+    got, nodes = _batched(engine, cuda, n, start, some[np.arange(num) % 37])
+    want, want_nodes = _plain(engine, cuda, n, start, some[np.arange(num) % 37])
+    assert (got == want).all()
+    assert nodes == want_nodes
+    _, first, _ = orc.sym_count_cases(n, start, some, None, threads=4)
+    assert (got[:37] == first[:num]).all()
