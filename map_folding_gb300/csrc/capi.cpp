@@ -449,10 +449,10 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
         if (d < 0) d = default_lunnon_depth(p->t);
         if (d > p->t.n) d = p->t.n;
         inst[k].table_offset = uint32_t(tables.size());
-        inst[k].n = p->t.n;
-        inst[k].dim = p->t.dim;
-        inst[k].start_leaf = d + 1;
-        inst[k].row = last_row(p->t);
+        inst[k].n = int16_t(p->t.n);
+        inst[k].dim = int16_t(p->t.dim);
+        inst[k].start_leaf = int16_t(d + 1);
+        inst[k].row = int16_t(last_row(p->t));
         tables.insert(tables.end(), p->t.next.begin(), p->t.next.end());
         tables.resize((tables.size() + 15) / 16 * 16, 0);
         states.emplace_back(p->t, d);
@@ -506,8 +506,8 @@ static int32_t lunnon_batch_impl(const mf_lunnon_plan *const *plans, int32_t num
     cudaEventRecord(tk.a, st);
     int max_levels = 0, row_levels = 0;
     for (const auto &I : inst) {
-        max_levels = std::max(max_levels, I.n - I.start_leaf);
-        if (I.row) row_levels = std::max(row_levels, I.n - I.start_leaf);
+        max_levels = std::max(max_levels, int(I.n) - I.start_leaf);
+        if (I.row) row_levels = std::max(row_levels, int(I.n) - I.start_leaf);
     }
     MF_TRY_CUDA(launch_lunnon_batched(d_meta, uint32_t(meta_used), uint32_t(tables.size()), num_plans,
                                       max_levels, row_levels, d_units,
@@ -711,7 +711,8 @@ int32_t mf_lunnon_batch_create(const mf_lunnon_plan *const *plans, int32_t num_p
         int d = depths ? depths[k] : -1;
         if (d < 0) d = default_lunnon_depth(p->t);
         if (d > p->t.n) d = p->t.n;
-        inst[k] = LunnonInstanceDev{uint32_t(meta.size()), p->t.n, p->t.dim, d + 1, last_row(p->t)};
+        inst[k] = LunnonInstanceDev{uint32_t(meta.size()), int16_t(p->t.n), int16_t(p->t.dim),
+                                    int16_t(d + 1), int16_t(last_row(p->t))};
         meta.insert(meta.end(), p->t.next.begin(), p->t.next.end());
         meta.resize((meta.size() + 15) / 16 * 16, 0);
         states.emplace_back(p->t, d);

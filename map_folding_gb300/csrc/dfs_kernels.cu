@@ -945,12 +945,13 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
             d_meta, mb, inst_offset, src, num, counts, nodes, Q, knobs.node_budget,             \
             knobs.wait_limit, shape.spread);                                                     \
     } while (0)
-    if (row_levels >= kRowLevels) {
-        // All the maps' tables are in every CTA's shared memory, so many small
-        // maps leave room for few CTAs: take the CTA size that keeps more
-        // warps on an SM.
-        const size_t warp = tail_bytes<false, 6>(32) + Carve<32, 17, 0>::kThreadBytes;
-        const size_t room = 227 * 1024;
+    // All the maps' tables are in every CTA's shared memory, so many small maps
+    // leave room for few CTAs: take the CTA size that keeps more warps on an SM.
+    // Where four warps' rows do not fit beside the tables (over 181 KB), the list
+    // search still does.
+    const size_t warp = tail_bytes<false, 6>(32) + Carve<32, 17, 0>::kThreadBytes;
+    const size_t room = 227 * 1024;
+    if (row_levels >= kRowLevels && mb + 4 * warp <= room) {
         const size_t small = room / (mb + 4 * warp + 1024) * 4;
         if (mb + 16 * warp <= room && small < 16) MF_LUN_BATCHED(512, 0, 6);
         else MF_LUN_BATCHED(128, 0, 6);

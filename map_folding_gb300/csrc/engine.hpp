@@ -209,13 +209,14 @@ uint64_t wide_workspace_bytes(uint64_t capacity);
 // Largest Lunnon map whose last row is counted on masks.
 constexpr int kRowLeaves = 41;
 
-// One Lunnon map as the batched kernel sees it.
+// One Lunnon map as the batched kernel sees it: 12 bytes, since every map of a
+// launch has one in shared memory.
 struct LunnonInstanceDev {
     uint32_t table_offset;  // into the concatenated next-tables
-    int32_t n;
-    int32_t dim;
-    int32_t start_leaf;
-    int32_t row;  // leaves of the last row of a 2-D map (0: no such row)
+    int16_t n;
+    int16_t dim;
+    int16_t start_leaf;
+    int16_t row;  // leaves of the last row of a 2-D map (0: no such row)
 };
 
 // d_edges: the 4 x 64 edge pages in device memory.

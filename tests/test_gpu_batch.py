@@ -46,3 +46,12 @@ def test_depths_per_instance(engine, cuda, golden):
     shapes = [(5, 5), (5, 5), (5, 5), (4, 4)]
     counts, _ = engine.lunnon_batch_count(shapes, depths=[0, 7, 20, 16])
     assert counts == [golden["lunnon"]["5x5"]] * 3 + [golden["lunnon"]["4x4"]]
+
+
+@pytest.mark.parametrize("small,many", [((2, 3), 1400), ((1, 3), 4250)])
+def test_many_small_maps_beside_one_with_rows(engine, cuda, golden, small, many):
+    """Tables that leave little shared memory: with 1,400 maps the rows' queues
+    just fit beside them, with 4,250 the list search alone does."""
+    counts, _ = engine.lunnon_batch_count([small] * many + [(5, 5)])
+    assert counts[:-1] == [{(2, 3): 60, (1, 3): 6}[small]] * many
+    assert counts[-1] == golden["lunnon"]["5x5"]

@@ -88,7 +88,7 @@ def _lunnon(host, maps, seed, rows=True):
         states.append(rec)
         owner += [k] * len(b)
     offset = len(meta)
-    meta += np.array(inst, np.int32).tobytes()
+    meta += np.array(inst, "<u4,<i2,<i2,<i2,<i2").tobytes()
     meta += bytes(-len(meta) % 16)
     meta = np.frombuffer(bytes(meta), np.uint8)
     states, owner = np.concatenate(states), np.array(owner, np.uint32)
