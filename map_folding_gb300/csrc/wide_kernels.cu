@@ -630,7 +630,15 @@ cudaError_t launch_wide_levels(const uint8_t *d_edges, int start_i, int last, co
     if (knobs.blocks_per_sm > 0 && int(knobs.blocks_per_sm) < fit) fit = int(knobs.blocks_per_sm);
     const int sms = device_sm_count();
     uint32_t spread = uint32_t(sms * fit * (kWideTPB / 32));
-    if (!kRow && last + 1 - start_i <= kShallow) spread = std::min(spread, uint32_t(sms * kShallowWarps));
+    // Shallow units as in the 64-bit kernel; those of six levels or less are done
+    // sooner than many warps have fetched theirs (3,000 of five / three levels with
+    // the first warps full, over ten warps an SM and over one: 34 / 30, 36 / 34 and
+    // 30 / 26 us; of six 36, 40 and over four 36; 30,000 of six 46, 42 and 51).
+    const uint64_t levels = last + 1 - start_i, sm = uint64_t(sms);
+    if (!kRow && levels <= kShallow) {
+        const uint64_t few = levels <= 5 ? sm : levels == 6 ? std::max(4 * sm, num / 16) : kShallowWarps * sm;
+        spread = uint32_t(std::min({uint64_t(spread), kShallowWarps * sm, few}));
+    }
     sym_wide_kernel<kWideTPB, LEVELS, kRow><<<unsigned(sms * fit), kWideTPB, smem, stream>>>(
         d_edges, start_i, last, d_cycles, record_bytes, num,
         reinterpret_cast<unsigned long long *>(d_counts),
