@@ -1355,12 +1355,13 @@ uint32_t mf_solve_cases(uint32_t n, uint32_t start_i, uint32_t stop_i, const uin
     std::vector<uint64_t> counts(case_count + 1);
     mf_run_stats st{};
     if (case_count) {
-        // The plain kernel is one launch and shares a case among 32 lanes; from
-        // 13 levels on a heavy case is worth more than a warp and the batched
-        // kernel splits it (64 / 256 7x7 cases of 14 cells, plain and batched:
-        // to 24 cells 292 / 458 and 485 / 769 us, to 26 519 / 899 and 607 /
-        // 805 us, to 28 1.70 / 4.12 and 1.09 / 1.72 ms).
-        const int mode = stop_i - start_i >= 13 ? 1 : 0;
+        // The plain kernel is one launch and shares a case among 32 lanes; a heavy
+        // case is worth more than a warp and the batched kernel splits it, the
+        // sooner the more cases there are.  Plain and batched, us: a 7x7 case of 14
+        // cells 12 levels on 254 / 342, 13 427 / 389, a 6x6 case of 16 403 / 356 and
+        // 549 / 391; 16 cases 10 levels on 466 / 675 and 304 / 668, 11 698 / 510 and
+        // 562 / 478; 256 cases 541 / 744 and 924 / 838, 798 / 704 and 2,336 / 963.
+        const int mode = stop_i - start_i >= (case_count < 8 ? 13u : 11u) ? 1 : 0;
         int rc = count_cases_host(int(n), int(start_i), int(stop_i), cycles.data(), case_count, mode,
                                   nullptr, counts.data(), &st, nullptr);
         if (rc) return write(0, 0, 3);

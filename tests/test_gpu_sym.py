@@ -173,6 +173,22 @@ def test_solve_cases_multiplier(engine, cuda, orc):
     assert status == 0 and count == total
 
 
+@pytest.mark.parametrize("n", [5, 7])
+@pytest.mark.parametrize("cases", [1, 7, 8, 256])
+@pytest.mark.parametrize("levels", [10, 11, 12, 13])
+def test_solve_cases_on_either_kernel(engine, cuda, orc, n, cases, levels):
+    """Numbers of cases and levels on both sides of where the kernel changes."""
+    raw = orc.sym_raw_prefixes(n, 8 if n == 5 else 13)
+    start = 8 if n == 5 else 13
+    cycles = raw[np.linspace(0, len(raw) - 1, cases).astype(int)]
+    buf = engine.pack_case_buffer(cycles, [1 + k % 3 for k in range(cases)], n)
+    count, nodes, status = engine.solve_cases(n, start, start + levels, buf, cases)
+    each = [orc.sym_count_to(n, c, start, start + levels) for c in cycles]
+    assert status == 0
+    assert count == sum(c * (1 + k % 3) for k, (c, _) in enumerate(each))
+    assert nodes == sum(w.nodes for _, w in each)
+
+
 def test_solve_cases_mfah_campaign(engine, cuda, orc, golden):
     """The bounded 7x7 campaign of mfah/README.md:59-68 through solve_cases,
     as its coordinator hands it out: the raw 14-cell prefixes in units of 64
