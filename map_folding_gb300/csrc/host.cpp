@@ -185,14 +185,23 @@ void expand_states(const LunnonTables &t, uint8_t *b, int from, int depth, F &&e
 // touches, to write.  Few states are kept from the first pass.
 LunnonStates::LunnonStates(const LunnonTables &t, int depth) : t_(t) {
     constexpr size_t kKept = 32768;
+    // Shallower where these would be many: they are held in memory, which the
+    // states themselves need not be (1x64 to depth 20: 122 MB with the
+    // 1,053,874 of depth 16, 3 MB with those of depth 13).
+    constexpr size_t kRoots = 65536;
     depth_ = std::min(std::max(depth, 0), t.n);
     split_ = std::max(0, std::min(depth_ - 4, t.n / 3 + 1));
-    uint8_t b[MF_MAX_LEAVES + 2] = {0};
     const size_t rec = size_t(t.n) + 1;
-    expand_states(t_, b, 0, split_, [&](const uint8_t *c) {
-        roots_.insert(roots_.end(), c, c + rec);
-        return true;
-    });
+    for (bool fit = false; !fit; split_ -= fit ? 0 : 3) {
+        uint8_t b[MF_MAX_LEAVES + 2] = {0};
+        roots_.clear();
+        expand_states(t_, b, 0, split_, [&](const uint8_t *c) {
+            fit = roots_.size() < kRoots * rec;
+            if (fit) roots_.insert(roots_.end(), c, c + rec);
+            return fit;
+        });
+        fit = fit || roots_.empty();  // no state at all
+    }
     const size_t roots = roots_.size() / rec;
     first_.assign(roots + 1, 0);
     each(0, roots, [&](size_t k, uint8_t *c, bool alone) {
@@ -231,9 +240,10 @@ void LunnonStates::each(size_t lo, size_t hi, F &&run) const {
         const double took = pool.empty() ? now_seconds() - start : 0;
         if (took > 3e-4 && took * double(hi - k - 1) > 2.5e-3 * double(k + 1 - lo)) {
             const size_t threads = std::min<size_t>({host_threads(), 16, (hi - k) / 4});
+            pool.reserve(threads);
             try {
                 for (size_t j = 1; j < threads; ++j) pool.emplace_back(help);
-            } catch (const std::system_error &) {  // no more threads: fewer do
+            } catch (const std::exception &) {  // no more threads or memory: fewer do
             }
         }
     }

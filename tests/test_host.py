@@ -186,3 +186,29 @@ def test_sym_fold_cli_queue_size_checked_in_stream_mode(engine):
                                      "Invalid MF_QUEUE_SIZE: abc"]
     env = dict(os.environ, MF_SETUP_ONLY="1", MF_QUEUE_SIZE="abc")  # not read before solving
     assert _cli("sym_fold", 7, 1, env=env).returncode == 0
+
+
+def test_counting_prefix_states_holds_few_of_them(engine):
+    """The 1e8 states of a 64-leaf strip at depth 20 are counted in a few MB."""
+    import subprocess
+    import sys
+
+    code = ("import re, map_folding_gb300 as mf\n"
+            "kb = lambda: int(re.search(r'VmHWM:\\s*(\\d+)', open('/proc/self/status').read())[1])\n"
+            "p = mf.LunnonPlan((1, 64)); p.count_prefixes(10); before = kb()\n"
+            "print(p.count_prefixes(20), kb() - before)")
+    out = subprocess.run([sys.executable, "-c", code], check=True, capture_output=True, text=True,
+                         cwd=Path(__file__).resolve().parent.parent).stdout.split()
+    assert int(out[0]) == 102511418
+    assert int(out[1]) < 32 * 1024
+
+
+def test_collected_ranges_of_many_states(engine, orc):
+    """Ranges of states whose shallower prefixes are too many to hold at first."""
+    import numpy as np
+
+    plan = engine.LunnonPlan((1, 64))
+    assert plan.count_prefixes(18) == 10274466
+    got = plan.collect(17)
+    _, want, _ = orc.lunnon_collect((1, 64), 17)
+    assert (got[:, :65] == want).all() and not got[:, 65:].any()
