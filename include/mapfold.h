@@ -61,7 +61,8 @@ typedef struct {
 /* Launch shape and scheduling knobs of the persistent (batched) kernels.
  * Zero in any field selects the built-in default. */
 typedef struct {
-    uint32_t block_threads;  /* threads per CTA: 128 or 256 */
+    uint32_t block_threads;  /* threads per CTA: 128 or 256 (not where a last row is
+                                counted on masks: see below) */
     uint32_t blocks_per_sm;  /* resident CTAs per SM (0: as many as fit) */
     uint32_t node_budget;    /* lockstep rounds (one node each) between split checks */
     uint32_t hungry_factor;  /* split while queued items < factor/8 x threads */
@@ -70,6 +71,11 @@ typedef struct {
     uint32_t stack_mode;     /* 0: DFS stack in shared memory when it fits, 1: local,
                                 2: sym counts on the 128-bit kernel whatever the board */
 } mf_batch_config;
+/* Where a last row is counted on masks the launch takes the CTA size that its
+ * shared memory leaves room for, and the stack is in local memory, whatever
+ * block_threads and stack_mode (0 or 1) say: squares of n >= 5 counted to the
+ * full board from above their last side, and Lunnon launches with a 2-D map of
+ * p1 >= 3, p2 >= 2 and at most 41 leaves that has four or more levels to go. */
 
 /* ======================================================================
  * Lunnon backtracking DFS over leaves (any dimension count, <= 64 leaves)

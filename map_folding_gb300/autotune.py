@@ -81,10 +81,28 @@ def _config(tpb: int, period: int, cap: int) -> BatchConfig:
     return c
 
 
+def lunnon_rows(shapes: Sequence[Sequence[int]], depths: Sequence[int]) -> bool:
+    """Whether a launch of these maps counts last rows on masks: it then takes
+    its own CTA size, whatever `block_threads` says (mf_batch_config)."""
+    for s, depth in zip(shapes, depths):
+        n = 1
+        for d in s:
+            n *= d
+        if len(s) == 2 and s[0] >= 3 and s[1] >= 2 and n <= 41 and n - depth - 1 >= 4:
+            return True
+    return False
+
+
+def sym_rows(n: int, start_i: int) -> bool:
+    """The same for full counts of an n x n board from `start_i` cells."""
+    return n >= 5 and start_i <= n * n - n
+
+
 def tune_lunnon_batch(shapes: Sequence[Sequence[int]], depth_offsets=(-2, 0, 2),
                       block_threads=(128, 256), periods=(32, 64, 128),
                       capacities=(1 << 16,), repeats: int = 2, use_cache: bool = True) -> dict:
     """Best configuration for counting all `shapes` in one batched launch.
+    Where the launch takes its own CTA size, `block_threads` is 0 and is not tried.
 
     Returns {"depths": [...], "block_threads", "node_budget", "queue_capacity",
     "seconds", "counts"}; every candidate's counts must agree (they are
@@ -104,7 +122,8 @@ def tune_lunnon_batch(shapes: Sequence[Sequence[int]], depth_offsets=(-2, 0, 2),
             for d in s:
                 n *= d
             depths.append(max(0, min(n, default_depth(s) + off)))
-        for tpb, period, cap in itertools.product(block_threads, periods, capacities):
+        sizes = (0,) if lunnon_rows(shapes, depths) else block_threads
+        for tpb, period, cap in itertools.product(sizes, periods, capacities):
             batch = api.LunnonBatch(shapes, depths, _config(tpb, period, cap))
             try:
                 times = []
@@ -131,7 +150,8 @@ def tune_lunnon_batch(shapes: Sequence[Sequence[int]], depth_offsets=(-2, 0, 2),
 def tune_sym(n: int, expanded_n: int, block_threads=(128, 256), periods=(32, 64, 128),
              repeats: int = 1, max_cases: int = 0, use_cache: bool = True) -> dict:
     """Best CTA size and bookkeeping period for a sym case set, timed with
-    graph replays on the device-resident cases."""
+    graph replays on the device-resident cases.  Where the launch takes its own
+    CTA size, `block_threads` is 0 and is not tried."""
     import numpy as np
     import torch
 
@@ -146,7 +166,8 @@ def tune_sym(n: int, expanded_n: int, block_threads=(128, 256), periods=(32, 64,
     d_counts = torch.zeros(len(cycles), dtype=torch.int64, device="cuda")
     best = None
     want = None
-    for tpb, period in itertools.product(block_threads, periods):
+    sizes = (0,) if sym_rows(n, plan.start_i) else block_threads
+    for tpb, period in itertools.product(sizes, periods):
         cfg = _config(tpb, period, 1 << 16)
         ws = torch.empty(api.sym_workspace_bytes(cfg), dtype=torch.uint8, device="cuda")
         g = api.SymGraph(n, plan.start_i, n * n, d_cyc.data_ptr(), len(cycles), d_counts.data_ptr(),

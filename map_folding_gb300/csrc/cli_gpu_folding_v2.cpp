@@ -5,8 +5,9 @@
 //
 // Argument checks, exit codes and output follow gpu_folding_v2.cu:544-699:
 // stdout is the decimal count only; stderr carries the key=value lines.
-// threads_per_block and blocks_per_sm shape the persistent kernel; batch
-// size, GPU count and queue depth are accepted and reported (one GPU, one
+// blocks_per_sm shapes the persistent kernel, threads_per_block too where no
+// row is counted on masks (grids of 2, 7 and 8, and searches of under four
+// levels); batch size, GPU count and queue depth are accepted and reported (one GPU, one
 // resident launch).  max_states > 0 counts only the first max_states prefix
 // states, as the reference's producer stops after them.  Grids are limited to
 // 8 (64 leaves) instead of the reference's 9.
