@@ -171,7 +171,6 @@ struct SymSource {
 struct LunnonSource {
     const uint8_t *states;
     const uint32_t *state_owner;
-    const LunnonInstanceDev *inst;
     uint32_t stride;
 };
 
@@ -193,7 +192,7 @@ struct LunnonSource {
 // accounting closed (leave_and_check).
 //
 // With TMAX > 0 a lane that comes to the last row (of up to TMAX cells) stops
-// there, and once kTailRoots lanes have (or no lane can go on) the warp counts
+// there, and once enough lanes have (count_rows_now) the warp counts
 // their rows together on masks (tail.cuh).
 template <int TPB, int WORDS, bool kSym, int TMAX, class Stk>
 __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
@@ -520,7 +519,8 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
         if constexpr (TMAX > 0) {
             const bool here = at_row();
             const unsigned at = __ballot_sync(kFull, here);
-            if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
+            bool walk = false;
+            if (count_rows_now(at, busy, here, row_level, walk)) {
                 const int K0 = last - eval;
                 uint32_t C = 0, counted = 0;
                 typename RowTail::Hist R = 0, H = 0;
@@ -553,6 +553,7 @@ __device__ __forceinline__ void persistent_loop(const uint8_t *s_tables,
                 __syncwarp();
                 round += kTailRounds;
             }
+            by_walk |= walk && here;
         }
         if (!bookkeeping) continue;
         round = 0;
@@ -926,7 +927,7 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
     cudaError_t e = cudaSuccess;
     const int sms = device_sm_count();
     const uint32_t mb = (meta_bytes + 15) / 16 * 16;
-    const LunnonSource src{d_states, d_state_owner, nullptr, lunnon_state_stride(64)};
+    const LunnonSource src{d_states, d_state_owner, lunnon_state_stride(64)};
     const int levels = pick_levels(max_levels, knobs.stack_mode == 1);
     auto *counts = reinterpret_cast<unsigned long long *>(d_counts);
     auto *nodes = reinterpret_cast<unsigned long long *>(d_nodes);

@@ -364,7 +364,8 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
         }
         const bool here = at_row();
         const unsigned at = __ballot_sync(kFull, here);
-        if (at && (__popc(at) >= kTailRoots || !__any_sync(kFull, busy && !here))) {
+        bool walk = false;
+        if (count_rows_now(at, busy, here, row_level, walk)) {
             uint32_t W[ServeTail::kRow] = {};
             uint32_t c = 0, counted = 0;
             ServeTail::Hist r = 0, h = 0;
@@ -396,6 +397,7 @@ __global__ void __launch_bounds__(TPB) serve_kernel(ServeArgs A) {
             __syncwarp();
             round += kTailRounds;
         }
+        by_walk |= walk && here;
         if (!bookkeeping) continue;
         round = 0;
         share_miss = false;

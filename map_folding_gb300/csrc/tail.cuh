@@ -588,6 +588,25 @@ constexpr int kRowSplit = 5;
 constexpr int kRowShare = 1;  // the same for a piece shared within the warp
 constexpr int kNoRow = 1 << 20;
 
+// Whether the lanes of `at`, which have come to their rows, are to be counted now
+// (all 32 lanes call): once kTailRoots of them have, or every busy lane that has a
+// row.  Beside lanes of maps without one, which never come, fewer than kFewRoots go
+// on by list (`walk`): a count stops the whole warp for some eight rounds, and a
+// root by list takes its own lane some 80.  Three 1x20 strips (4.1 ms by themselves)
+// and five 4x6 maps (1.1) in one launch: 17.6 ms waiting for all busy lanes, 7.0 so;
+// a batch of 64 maps, half its work strips: 12.9 and 8.0 ms (8.4 with 4 or 16 roots
+// and counting once seven of eight lanes with rows have come).
+constexpr int kFewRoots = 8;
+__device__ __forceinline__ bool count_rows_now(unsigned at, bool busy, bool here, int row_level,
+                                               bool &walk) {
+    walk = false;
+    if (!at) return false;
+    const int come = __popc(at);
+    if (come < kTailRoots && __any_sync(kFull, busy && !here && row_level != kNoRow)) return false;
+    walk = come < kFewRoots && __any_sync(kFull, busy && row_level == kNoRow);
+    return !walk;
+}
+
 // The pages of the last row of a square: the row's last cell is `last`, held
 // by last - 1 and by a cell of the row before.  `stride` cells per page.
 __device__ __forceinline__ TailPages sym_row_pages(const uint8_t *edge, int last, int stride) {

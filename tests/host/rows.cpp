@@ -126,7 +126,7 @@ extern "C" int32_t host_lunnon(const uint8_t *meta, uint32_t bytes, uint32_t ins
     std::vector<TaskRecord> slots(Ring::kCells);
     Ring ring(slots.data());
     watch(ring.hdr, counts, maps, at_leave);
-    const LunnonSource src{states, owner, nullptr, stride};
+    const LunnonSource src{states, owner, stride};
     if (rows) run_lunnon<6>(meta, bytes, inst_offset, src, num, counts, nodes, ring.q, seed);
     else run_lunnon<0>(meta, bytes, inst_offset, src, num, counts, nodes, ring.q, seed);
     return int32_t(ring.hdr.error);

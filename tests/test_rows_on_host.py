@@ -257,3 +257,20 @@ def test_long_counts_go_on_in_64_bits(tmp_path, orc):
     test_square_rows(host, orc, 8, 57, 40, 2)
     test_9x9_rows(host, 70)
     test_9x9_rows(host, 74)
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+@pytest.mark.parametrize("strips", [1, 6, 30])
+def test_rows_beside_maps_without(host, orc, strips, seed):
+    """Few and many lanes of a warp on maps that have no row: the others' rows are
+    counted without them, a few roots by list."""
+    maps, want, nodes = [], [], 0
+    for dims, depth, most in (((1, 13), 5, strips), ((5, 4), 10, 40), ((2, 2, 3), 4, strips), ((7, 2), 6, 30)):
+        a, b, _ = orc.lunnon_collect(dims, depth)
+        total, _, w = orc.lunnon_resume_many(dims, depth + 1, a[:most], b[:most])
+        maps.append((dims, depth, b[:most]))
+        want.append(total)
+        nodes += w.nodes
+    got, got_nodes, left = _lunnon(host, maps, seed)
+    assert list(got) == want and got_nodes == nodes
+    assert left == got.sum()
