@@ -474,6 +474,22 @@ __device__ __forceinline__ bool share_in_warp(const List &L, Stk &S, bool search
 constexpr int kShareLanes = 2;
 constexpr int kMinShareHeight = 2;
 
+// Square units of at most kShallow levels searched by list are spread over ten warps
+// an SM and no more: a warp runs as long as its longest unit, so fuller warps take
+// fewer instructions in all, and ten an SM cover the latencies (100,000 7x7 units
+// from 44 cells: 118.8 us with the first warps full, 152.4 spread over all 24 an SM,
+// 110.5 over ten; 2,000: 77, 60, 60; of 8 levels 100,000 and 12,000: 716, 647, 550
+// and 535, 289, 277; of 9 on 8x8, 12,000: 1,442, 574, 581).
+constexpr int kShallow = 7;
+constexpr int kShallowWarps = 10;
+
+// The plain kernels share among as many idle lanes below that depth, and not at
+// all in units of at most kNoShare levels, which are over too soon (400,000 7x7
+// units of 40 cells, three levels / six: 77.5 / 984 us without sharing, 97 / 737
+// from two idle lanes, 90 / 667 from eight).
+constexpr int kShareLanesShallow = 8;
+constexpr int kNoShare = 3;
+
 // Run the loaded units of a warp to completion in lockstep rounds (no refill):
 // the plain kernels.  A lane whose unit is done takes pieces of the others',
 // so the heaviest unit of a warp no longer sets its time; `acc` holds 32
@@ -497,11 +513,35 @@ __device__ __forceinline__ unsigned long long run_units(const Rules &R, const Li
     }
     bool walking = false, miss = false;
     typename Rules::Walk w;
+    auto step = [&]() {
+        if (!busy) return;
+        if (!walking) {
+            R.begin(L, eval, nodes, w);
+            walking = true;
+        }
+        if (!R.run(L, w, kWalkCap)) return;
+        walking = false;
+        const uint64_t g = R.result(w, nodes);
+        eval = apply_advance(L, S, lvl, eval, root, last, fresh, g, leaves);
+        fresh = false;
+        busy = eval >= 0;
+        if (!busy) {
+            if (owner == lane) own += leaves;
+            else if (leaves) atomicAdd(acc + owner, leaves);
+            leaves = 0;
+        }
+    };
+    const int levels = last + 1 - root;  // the same for all units
+    if (levels <= kNoShare) {
+        while (__any_sync(kFull, busy)) step();
+        return own;
+    }
+    const int enough = levels <= kShallow ? kShareLanesShallow : kShareLanes;
     for (int round = 0;; ++round) {
         const unsigned idle = __ballot_sync(kFull, !busy);
         if (idle == kFull) break;
         if (!(round & 15)) miss = false;
-        if (__popc(idle) >= kShareLanes && !miss) {
+        if (__popc(idle) >= enough && !miss) {
             int whose = 0;
             miss = !share_in_warp(
                 L, S, busy && !fresh, root, lvl, last - kMinShareHeight, idle,
@@ -516,24 +556,7 @@ __device__ __forceinline__ unsigned long long run_units(const Rules &R, const Li
                     busy = true;
                 });
         }
-        if (busy) {
-            if (!walking) {
-                R.begin(L, eval, nodes, w);
-                walking = true;
-            }
-            if (R.run(L, w, kWalkCap)) {
-                walking = false;
-                const uint64_t g = R.result(w, nodes);
-                eval = apply_advance(L, S, lvl, eval, root, last, fresh, g, leaves);
-                fresh = false;
-                busy = eval >= 0;
-                if (!busy) {
-                    if (owner == lane) own += leaves;
-                    else if (leaves) atomicAdd(acc + owner, leaves);
-                    leaves = 0;
-                }
-            }
-        }
+        step();
     }
     __syncwarp();
     return own + acc[lane];
@@ -760,15 +783,6 @@ constexpr int kWarpTake = 8;
 // counted by itself (with sharing within the warp, 4 / 6: 1x16 at depth 10 254 /
 // 230 us, 2x10 at 12 448 / 425 us).
 constexpr int kMinRingHeight = 6;
-
-// Square units of at most kShallow levels searched by list are spread over ten warps
-// an SM and no more: a warp runs as long as its longest unit, so fuller warps take
-// fewer instructions in all, and ten an SM cover the latencies (100,000 7x7 units
-// from 44 cells: 118.8 us with the first warps full, 152.4 spread over all 24 an SM,
-// 110.5 over ten; 2,000: 77, 60, 60; of 8 levels 100,000 and 12,000: 716, 647, 550
-// and 535, 289, 277; of 9 on 8x8, 12,000: 1,442, 574, 581).
-constexpr int kShallow = 7;
-constexpr int kShallowWarps = 10;
 
 // How many split items a warp with work is to give now, of a launch of `num`
 // units and `warps` warps: its share of what is wanted, twice over.  Every

@@ -780,10 +780,14 @@ cudaError_t reset_queue(const Queue &Q, uint64_t *counts, uint64_t words, cudaSt
 
 }  // namespace
 
-// Units per warp of a plain launch of CTAs of `tpb` threads, `bpsm` of them
-// resident on an SM.
-static int plain_units_per_warp(uint64_t num, int bpsm, int tpb) {
-    const uint64_t warps = uint64_t(device_sm_count()) * uint64_t(bpsm) * uint64_t(tpb / 32);
+// Units per warp of a plain launch of units of `levels` levels on CTAs of `tpb`
+// threads, `bpsm` of them resident on an SM: spread over all resident warps, shallow
+// ones over ten an SM (see kShallow), and where lanes do not share 32 each.
+static int plain_units_per_warp(uint64_t num, int bpsm, int tpb, int levels) {
+    if (levels <= kNoShare) return 32;
+    const uint64_t sms = uint64_t(device_sm_count());
+    uint64_t warps = sms * uint64_t(bpsm) * uint64_t(tpb / 32);
+    if (levels <= kShallow && warps > sms * kShallowWarps) warps = sms * kShallowWarps;
     const uint64_t k = (num + warps - 1) / (warps ? warps : 1);
     return k < 1 ? 1 : (k > 32 ? 32 : int(k));
 }
@@ -803,7 +807,7 @@ cudaError_t launch_sym_plain(const uint8_t *d_edges, int start_i, int stop_i,
         const size_t smem = tables + Carve<TPB, 16, LV>::kThreadBytes + 8 * TPB;                \
         cudaError_t e = prepare(sym_plain_kernel<TPB, LV>, smem, TPB, 0, bpsm);                 \
         if (e != cudaSuccess) return e;                                                         \
-        const int per = plain_units_per_warp(num, bpsm, TPB);                                   \
+        const int per = plain_units_per_warp(num, bpsm, TPB, stop_i - start_i);                 \
         const uint64_t blocks = (num + per * (TPB / 32) - 1) / (per * (TPB / 32));              \
         sym_plain_kernel<TPB, LV><<<unsigned(blocks), TPB, smem, stream>>>(                     \
             d_edges, start_i, stop_i, d_cycles, num, per, counts, nodes);                       \
@@ -835,7 +839,7 @@ cudaError_t launch_lunnon_plain(const uint8_t *d_table, int n, int dim, int star
         const size_t smem = table_bytes + Carve<TPB, 17, LV>::kThreadBytes + 8 * TPB;           \
         cudaError_t e = prepare(lunnon_plain_kernel<TPB, LV>, smem, TPB, 0, bpsm);              \
         if (e != cudaSuccess) return e;                                                         \
-        const int k = plain_units_per_warp(num, bpsm, TPB);                                     \
+        const int k = plain_units_per_warp(num, bpsm, TPB, n + 1 - start_leaf);                 \
         const uint64_t blocks = (num + k * (TPB / 32) - 1) / (k * (TPB / 32));                  \
         lunnon_plain_kernel<TPB, LV><<<unsigned(blocks), TPB, smem, stream>>>(                  \
             d_table, table_bytes, n, dim, start_leaf, d_states, stride, num, k, per, tot,       \

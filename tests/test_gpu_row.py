@@ -113,3 +113,20 @@ def test_many_shallow_units(engine, cuda, orc, n, start, num):
     assert nodes == want_nodes
     _, first, _ = orc.sym_count_cases(n, start, some, None, threads=4)
     assert (got[:37] == first[:num]).all()
+
+
+@pytest.mark.parametrize("n,start", [(5, 19), (7, 43)])
+@pytest.mark.parametrize("levels", [1, 3, 4, 6])
+@pytest.mark.parametrize("num", [1, 33, 1521, 20000])
+def test_plain_units_of_a_few_levels(engine, cuda, orc, n, start, levels, num):
+    """Where the plain kernel begins to share, and how it spreads such units."""
+    rng = np.random.default_rng([n, start, levels])
+    root = np.zeros(64, np.uint8)
+    root[:3] = (1, 2, 0)
+    some = np.array([_descend(orc, n, root, 3, start, rng) for _ in range(37)])
+    want = np.array([orc.sym_count_to(n, c, start, start + levels)[0] for c in some], np.uint64)
+    d = cuda.from_numpy(np.ascontiguousarray(some[np.arange(num) % 37])).cuda()
+    counts = cuda.full((num,), 7, dtype=cuda.int64, device="cuda")
+    engine.count_cases_device(n, start, start + levels, d.data_ptr(), num, counts.data_ptr())
+    cuda.cuda.synchronize()
+    assert (counts.cpu().numpy().view(np.uint64) == want[np.arange(num) % 37]).all()
