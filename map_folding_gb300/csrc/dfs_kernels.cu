@@ -739,6 +739,12 @@ std::atomic<uint32_t> g_inject{0};
 
 __global__ void phantom_ticket_kernel(QueueHeader *hdr) { hdr->spawn_tail = 1; }
 
+// Levels below the first of map units that are spread as shallow squares' are
+// (37,378 states of 1x16 three levels from the end: 109 us over all warps, 87 over
+// ten an SM; 40,000 of 1x18 four levels 229 and 203; of five over all 409, with the
+// first warps full 470).
+constexpr int kShallowMaps = 3;
+
 // Launch size of a persistent launch over `units` initial units searched
 // `levels` levels deep: the whole resident grid, or -- for a small job, whose
 // units are shallow (at most 10 levels to go, so none of them is heavy) --
@@ -754,7 +760,7 @@ struct LaunchShape {
 };
 
 LaunchShape persistent_shape(int sms, int bpsm, int tpb, uint64_t units, int levels,
-                             uint64_t ring_knob, bool square_list = false) {
+                             uint64_t ring_knob, int shallow) {
     const uint64_t full = uint64_t(sms) * uint64_t(bpsm);
     if (levels > 10) return LaunchShape{unsigned(full), ring_knob, uint32_t(full * (tpb / 32))};
     const uint64_t warps = (units + 3) / 4;
@@ -764,7 +770,7 @@ LaunchShape persistent_shape(int sms, int bpsm, int tpb, uint64_t units, int lev
     uint64_t ring = 1024;
     while (ring < 2 * blocks * uint64_t(tpb) && ring < ring_knob) ring <<= 1;
     uint64_t spread = blocks * per_block;
-    if (square_list && levels <= kShallow && spread > uint64_t(sms) * kShallowWarps)
+    if (levels <= shallow && spread > uint64_t(sms) * kShallowWarps)
         spread = uint64_t(sms) * kShallowWarps;
     return LaunchShape{unsigned(blocks), ring < ring_knob ? ring : ring_knob, uint32_t(spread)};
 }
@@ -884,7 +890,7 @@ cudaError_t launch_sym_batched(const uint8_t *d_edges, int n, int start_i, int s
         if (e != cudaSuccess) return e;                                                          \
         const LaunchShape shape =                                                                \
             persistent_shape(sms, bpsm, TPB, num, stop_i - start_i, knobs.queue_capacity,        \
-                             TM == 0);                                                           \
+                             TM == 0 ? kShallow : 0);                                            \
         const Queue Q = carve_queue(d_workspace, shape.ring);                                    \
         e = reset_queue(Q, d_counts, num + own_nodes, stream);                                   \
         if (e != cudaSuccess) return e;                                                          \
@@ -942,7 +948,8 @@ cudaError_t launch_lunnon_batched(const uint8_t *d_meta, uint32_t meta_bytes, ui
         e = prepare(lunnon_batched_kernel<TPB, LV, TM>, smem, TPB, knobs.blocks_per_sm, bpsm);   \
         if (e != cudaSuccess) return e;                                                          \
         const LaunchShape shape =                                                                \
-            persistent_shape(sms, bpsm, TPB, num, max_levels, knobs.queue_capacity);             \
+            persistent_shape(sms, bpsm, TPB, num, max_levels, knobs.queue_capacity,              \
+                             TM == 0 ? kShallowMaps : 0);                                        \
         const Queue Q = carve_queue(d_workspace, shape.ring);                                    \
         e = reset_queue(Q, d_counts, words, stream);                                             \
         if (e != cudaSuccess) return e;                                                          \
