@@ -87,7 +87,7 @@ struct Scratch {
 std::recursive_mutex g_scratch_mu;
 Scratch g_scratch[8];
 
-enum Slot { kDevUnits = 0, kDevCounts, kDevWork, kDevAux, kHostUnits, kHostCounts, kDevAux2, kSlots };
+enum Slot { kDevUnits = 0, kDevCounts, kDevWork, kHostUnits, kHostCounts, kSlots };
 
 void *scratch(int slot, size_t bytes, bool pinned) {
     Scratch &s = g_scratch[slot];

@@ -80,13 +80,6 @@ struct TailLayout {
     static constexpr int kBytes = ((kEnd > kScratchEnd ? kEnd : kScratchEnd) + 127) / 128 * 128;
 };
 
-// 1 << k, 0 for k >= 32.
-__device__ __forceinline__ uint32_t bit32(uint32_t k) {
-    uint32_t r;
-    asm("shl.b32 %0, %1, %2;" : "=r"(r) : "r"(1u), "r"(k));
-    return r;
-}
-
 // The row's pages: partner tables of the placed cells (an entry >= the
 // number of placed cells: none).
 struct TailPages {

@@ -273,10 +273,10 @@ __device__ __forceinline__ void wide_put(uint4 *slots, const Queue &Q, unsigned 
 // 128-bit masks: initial units by a warp-aggregated atomicAdd, lockstep
 // rounds, bookkeeping every `period` rounds (idle-lane report, donation of
 // the shallowest untried siblings while lanes wait), split items taken by
-// Split record: list words 0..kWideWords-1, owner, untried mask (4 words),
-// level, whether the row may be counted on masks.
 // idle lanes, and the same leaving rule; lanes of a warp share as there.  With
-// kRow the 9x9 board's last row is counted on masks (tail.cuh).
+// kRow the 9x9 board's last row is counted on masks (tail.cuh).  Split record: list
+// words 0..kWideWords-1, owner, untried mask (4 words), level, whether the row may
+// be counted on masks.
 template <int TPB, int LEVELS, bool kRow>
 __global__ void __launch_bounds__(TPB)
     sym_wide_kernel(const uint8_t *__restrict__ edges, int start_i, int last,
