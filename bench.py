@@ -7,7 +7,7 @@ completion, i.e. the whole 7x7 answer 129950723279272, with the batched
 persistent work-stealing kernel.  Inputs are resident in HBM for `value`;
 `e2e` runs the same count through the C ABI with host buffers (case
 selection, host->device copy, kernel, device->host copy of per-case counts).
-After the timed steps, on one GPU: the plain one-thread-per-case kernel
+After the timed steps, on one GPU: the plain one-case-per-lane kernel
 counts the same cases once (`batched_vs_plain`), and the serving stream's
 8x8 chunks run through the request server (`serving`: chunk p50/p99, each
 chunk checked against the reference's count).
@@ -42,8 +42,8 @@ UNIT = "nodes/s"
 
 
 # DRAM bytes per case of the batched kernel: read + write of the ncu capture
-# of the first 20,000 7x7 cases (15.83 + 13.39 MB), per case.
-TRAFFIC_PER_CASE = (15_830_000 + 13_390_000) / 20_000
+# of the first 20,000 7x7 cases (15.81 + 13.27 MB), per case.
+TRAFFIC_PER_CASE = (15_810_560 + 13_268_736) / 20_000
 
 # Issue profile of the batched kernel over one whole 7x7 count (one ncu pass
 # over a full launch of this bench's workload,
@@ -54,10 +54,10 @@ TRAFFIC_PER_CASE = (15_830_000 + 13_390_000) / 20_000
 # warp-instruction issue rate against the SMs' issue ceiling.  The ALU-pipe
 # share comes from the fuller capture of the first 20,000 cases
 # (profiles/sym_batched_7x7_first20k.md).
-ISSUE_PROFILE = {"warp_inst_per_node": 5_054_012_679_255 / 556_214_135_282,
-                 "lanes_per_inst": 128_393_196_038_274 / 5_054_012_679_255,
-                 "issue_active": 5_054_012_679_255 / 8_566_662_475_394,
-                 "alu_pipe_first20k": 0.600,
+ISSUE_PROFILE = {"warp_inst_per_node": 5_063_030_191_748 / 556_214_135_282,
+                 "lanes_per_inst": 128_696_253_217_823 / 5_063_030_191_748,
+                 "issue_active": 5_063_030_191_748 / 8_671_154_979_794,
+                 "alu_pipe_first20k": 0.595,
                  "source": "profiles/sym_batched_7x7_full_count.md"}
 
 
@@ -68,9 +68,9 @@ def work_counts() -> dict:
     return json.loads(p.read_text()).get("7x7_d24_all", {}) if p.exists() else {}
 
 
-def issue_figures(nodes_per_step: int, t_step: float, clock_summary: dict) -> dict:
-    """Issue-slot view of the DFS kernel: chain steps (get_good walk
-    iterations) per second and per SMSP issue slot at the sampled SM clock."""
+def issue_figures(nodes_per_step: int, clock_summary: dict) -> dict:
+    """The clock that the issue figures go by, and whether the nodes counted
+    are the oracle's."""
     import torch
 
     work = work_counts()
@@ -79,11 +79,6 @@ def issue_figures(nodes_per_step: int, t_step: float, clock_summary: dict) -> di
     out = {"sms": sms, "sm_mhz": mhz, "nodes_match_oracle": None}
     if work.get("steps"):
         out["nodes_match_oracle"] = work.get("nodes") == nodes_per_step
-        steps_s = work["steps"] / t_step
-        out["chain_steps_per_s"] = steps_s
-        out["chain_steps_per_step"] = work["steps"]
-        if mhz:
-            out["chain_steps_per_issue_slot"] = steps_s / (sms * 4 * mhz * 1e6)
     return out
 
 
@@ -115,7 +110,7 @@ def issue_roofline(cases: int, nodes_per_step: int, t_step: float, clock_summary
         "hbm": {"achieved": hbm_achieved, "peak": hbm_peak, "unit": "GB/s",
                 "frac": hbm_achieved / hbm_peak, "peak_source": peak_kind,
                 "algorithmic_bytes": algo_bytes},
-        "issue": issue_figures(nodes_per_step, t_step, clock_summary),
+        "issue": issue_figures(nodes_per_step, clock_summary),
     }
 
 
@@ -447,8 +442,8 @@ def run_ours(args):
         e2e_st = st
     e2e_value = world * nodes_per_step * len(e2e_times) / sum(e2e_times)
 
-    # The plain one-thread-per-case kernel on the same cases, once (single
-    # GPU only: its ~430 s would hold the other ranks at the final barrier).
+    # The plain one-case-per-lane kernel on the same cases, once (single
+    # GPU only: its ~76 s would hold the other ranks at the final barrier).
     plain_s = None
     if args.plain and world == 1:
         a = torch.cuda.Event(enable_timing=True)
@@ -986,8 +981,8 @@ def main():
     ap.add_argument("--steps", type=int, default=3)
     ap.add_argument("--warmup", type=int, default=3)
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
-    # The plain one-thread-per-case kernel needs ~430 s for the 7x7 count (its
-    # heaviest case runs on one thread); it runs once, after the timed steps.
+    # The plain one-case-per-lane kernel needs ~76 s for the 7x7 count (its
+    # heaviest cases run on one warp each); it runs once, after the timed steps.
     ap.add_argument("--plain", action="store_true", default=True)
     ap.add_argument("--no-plain", dest="plain", action="store_false")
     ap.add_argument("--no-serving", dest="serving", action="store_false", default=True,
